@@ -74,6 +74,7 @@ struct Resident {
     bool coeffs_valid = false;
     DevBuf psi[2][3][4];     // CPML accumulators per set and axis
     DevBuf tab[3][6];
+    DevBuf xtab[6], yztab[2], tables, work;   // tables of the fused step (MarchArgs)
     DevBuf snap[2][6];
     DevBuf stage;            // complex128 staging (one component)
     std::vector<DevBuf> src_ap;    // per source: 6 comps of amp/phase (complex128)
@@ -88,6 +89,9 @@ struct Resident {
         for (int c = 0; c < 3; c++) { bE[c].release(); aE[c].release(); bH[c].release(); }
         for (auto& s : psi) for (auto& a : s) for (auto& b : a) b.release();
         for (auto& a : tab) for (auto& b : a) b.release();
+        for (auto& b : xtab) b.release();
+        for (auto& b : yztab) b.release();
+        tables.release(); work.release();
         for (auto& s : snap) for (auto& b : s) b.release();
         stage.release();
         for (auto& b : src_ap) b.release();
@@ -777,24 +781,58 @@ template <typename T> Resident<T>& resident(FDTDHandle* h);
 template <> Resident<float>& resident<float>(FDTDHandle* h) { return h->r32; }
 template <> Resident<double>& resident<double>(FDTDHandle* h) { return h->r64; }
 
+// x-slab state rows of the fused step (MarchArgs): whole 16-byte vectors.
+struct XSlab {
+    int pitch = 0, max_slot = 0;
+    bool ok = false;         // no vector holds cells of both x slabs
+};
+
+template <typename T>
+XSlab x_slab(const FDTDHandle* h) {
+    constexpr int V = 16 / (int)sizeof(T);
+    auto up = [](int x) { return (x + V - 1) / V * V; };
+    XSlab s;
+    const int w0 = up(h->w[0]), first = (h->Nx - h->w[1]) & ~(V - 1);
+    s.ok = h->w[0] >= 0 && h->w[1] >= 0 && (h->w[0] == 0 || h->w[1] == 0 || w0 <= first);
+    s.max_slot = w0 - first;
+    s.pitch = w0 + (h->w[1] > 0 ? up(h->Nx) - first : 0);
+    return s;
+}
+
+// Can the fused step take this grid?  Non-periodic boundaries, 32-bit byte
+// offsets in every array, x slabs that share no vector.
+template <typename T>
+bool march_possible(const FDTDHandle* h) {
+    for (int a = 0; a < 3; a++)
+        if (h->bc[a] != '0' && h->bc[a] != 'E' && h->bc[a] != 'H') return false;
+    for (int q = 0; q < 6; q++)
+        if (h->w[q] < 0) return false;
+    const long long px = (h->Nx + 31) / 32 * 32, lim = std::min(1LL << 31, (1LL << 32) / (long long)sizeof(T));
+    const XSlab x = x_slab<T>(h);
+    return x.ok && h->Nz * (h->Ny * px) < lim && h->Nz * ((long long)h->Ny * x.pitch) < lim &&
+           h->Nz * ((h->w[2] + h->w[3]) * px) < lim && (h->w[4] + h->w[5]) * (h->Ny * px) < lim;
+}
+
 // Allocates the resident arrays for the current grid and PML widths.
+// march: the arrays of the fused step (a second set of the fields and of the
+// H-update CPML state, whole-vector x-slab rows).
 // halo = 1 (z slabs): the six field arrays get one plane below and one above
 // the slab; the interior starts one plane into each array.
 template <typename T>
-int alloc_resident(FDTDHandle* h, Resident<T>& r, bool two_sets, int halo = 0) {
+int alloc_resident(FDTDHandle* h, Resident<T>& r, bool march, int halo = 0) {
     int px = (h->Nx + 31) / 32 * 32;
     bool same = r.Nx == h->Nx && r.Ny == h->Ny && r.Nz == h->Nz && r.px == px && r.halo == halo;
     if (!same) r.release_all();
     r.Nx = h->Nx; r.Ny = h->Ny; r.Nz = h->Nz; r.px = px; r.halo = halo;
     size_t cells = (size_t)h->Nz * h->Ny * px;
     size_t fcells = (size_t)(h->Nz + 2 * halo) * h->Ny * px;
-    long long slab[3] = {(long long)h->Nz * h->Ny * (h->w[0] + h->w[1]),
+    long long slab[3] = {(long long)h->Nz * h->Ny * (march ? x_slab<T>(h).pitch : h->w[0] + h->w[1]),
                          (long long)h->Nz * (h->w[2] + h->w[3]) * px,
                          (long long)(h->w[4] + h->w[5]) * h->Ny * px};
-    for (int s = 0; s < (two_sets ? 2 : 1); s++) {
+    for (int s = 0; s < (march ? 2 : 1); s++) {
         for (int c = 0; c < 6; c++) CK(r.F[s][c].ensure(sizeof(T) * fcells));
         for (int a = 0; a < 3; a++)
-            for (int q = 0; q < 4; q++) CK(r.psi[s][a][q].ensure(sizeof(T) * (slab[a] ? slab[a] : 1)));
+            for (int q = 0; q < (s ? 2 : 4); q++) CK(r.psi[s][a][q].ensure(sizeof(T) * (slab[a] ? slab[a] : 1)));
     }
     for (int c = 0; c < 3; c++) CK(r.bE[c].ensure(sizeof(T) * cells));
     for (int s = 0; s < 2; s++)
@@ -848,7 +886,16 @@ int prepare_materials(FDTDHandle* h, Resident<T>& r) {
             CK(cudaGetLastError());
         }
     }
-    // CPML tables reordered by local slab index (min slab reversed) with 1/kappa
+    // CPML tables reordered by local slab index (min slab reversed) with 1/kappa,
+    // and the forms the fused step reads (MarchArgs); one upload for all of them
+    using Dup = typename fdtdb::pk::DupOf<T>::type;
+    std::vector<unsigned char> host;
+    std::vector<std::pair<DevBuf*, size_t>> place;
+    auto put = [&](DevBuf& b, const void* p, size_t bytes) {
+        place.push_back({&b, host.size()});
+        host.insert(host.end(), (const unsigned char*)p, (const unsigned char*)p + bytes);
+        host.resize((host.size() + 255) / 256 * 256);
+    };
     for (int a = 0; a < 3; a++) {
         int w0 = h->w[2 * a], w1 = h->w[2 * a + 1];
         std::vector<T> t[6];
@@ -862,12 +909,30 @@ int prepare_materials(FDTDHandle* h, Resident<T>& r) {
             t[4][l] = T(h->tab[a][4][tq]);
             t[5][l] = T(h->tab[a][5][tq]);
         }
-        for (int q = 0; q < 6; q++) {
-            CK(r.tab[a][q].ensure(sizeof(T) * t[q].size()));
-            CK(cudaMemcpyAsync(r.tab[a][q].p, t[q].data(), sizeof(T) * t[q].size(),
-                               cudaMemcpyDefault, h->stream));
+        for (int q = 0; q < 6; q++) put(r.tab[a][q], t[q].data(), sizeof(T) * t[q].size());
+        if (a == 0) {
+            std::vector<T> row(r.px);
+            for (int q = 0; q < 6; q++) {
+                for (int k = 0; k < r.px; k++) {
+                    const int l = k < w0 ? k : (k >= h->Nx - w1 && k < h->Nx) ? w0 + k - (h->Nx - w1) : -1;
+                    row[k] = l >= 0 ? t[q][l] : T(q % 3 == 0 ? 1 : 0);
+                }
+                put(r.xtab[q], row.data(), sizeof(T) * row.size());
+            }
+        } else {
+            std::vector<Dup> d(6 * t[0].size());
+            for (size_t l = 0; l < t[0].size(); l++)
+                for (int q = 0; q < 6; q++) d[6 * l + q] = fdtdb::pk::DupOf<T>::make(t[q][l]);
+            put(r.yztab[a - 1], d.data(), sizeof(Dup) * d.size());
         }
-        CK(cudaStreamSynchronize(h->stream));
+    }
+    CK(r.tables.ensure(host.size()));
+    CK(cudaMemcpyAsync(r.tables.p, host.data(), host.size(), cudaMemcpyDefault, h->stream));
+    CK(cudaStreamSynchronize(h->stream));
+    for (auto& q : place) {
+        q.first->release();
+        q.first->p = (unsigned char*)r.tables.p + q.second;
+        q.first->owned = false;
     }
     r.coeffs_valid = true;
     return FDTD_OK;
@@ -967,6 +1032,38 @@ fdtdb::GridView<T> make_view(FDTDHandle* h, Resident<T>& r, int set = 0) {
     return g;
 }
 
+// The fused step's view of the resident state: reads field set `set`.
+template <typename T>
+int make_march(FDTDHandle* h, Resident<T>& r, int set, bool src_general, fdtdb::MarchArgs<T>& a) {
+    a.g = make_view<T>(h, r, 0);
+    for (int c = 0; c < 6; c++) {
+        a.in.c[c] = dptr<T>(r.F[set][c]);
+        a.out.c[c] = dptr<T>(r.F[1 - set][c]);
+        a.xtab[c] = dptr<T>(r.xtab[c]);
+    }
+    for (int x = 0; x < 3; x++)
+        for (int q = 0; q < 2; q++) {
+            a.ph_in[x][q] = dptr<T>(r.psi[set][x][q]);
+            a.ph_out[x][q] = dptr<T>(r.psi[1 - set][x][q]);
+            a.pe[x][q] = dptr<T>(r.psi[0][x][2 + q]);
+        }
+    const XSlab x = x_slab<T>(h);
+    a.ytab = dptr<typename fdtdb::pk::DupOf<T>::type>(r.yztab[0]);
+    a.ztab = dptr<typename fdtdb::pk::DupOf<T>::type>(r.yztab[1]);
+    const T od[3] = {a.g.odx, a.g.ody, a.g.odz};
+    for (int c = 0; c < 3; c++) {
+        a.o[c] = fdtdb::pk::DupOf<T>::make(od[c]);
+        a.m[c] = fdtdb::pk::DupOf<T>::make(a.g.bH[c]);
+    }
+    a.mone = fdtdb::pk::DupOf<T>::make(T(-1));
+    a.x_pitch = x.pitch;
+    a.x_max_slot = x.max_slot;
+    a.src_general = src_general ? 1 : 0;
+    a.err = dptr<int>(r.err);
+    CK(fdtdb::march_maps<T>(a));
+    return FDTD_OK;
+}
+
 // Probe point -> offset into the pitched E arrays.  Probe indices address the
 // padded local arrays of the reference; a probe on a face ghost reads the
 // periodic copy that the one-rank ghost exchange leaves there
@@ -1024,27 +1121,38 @@ int solve_impl(FDTDHandle* h, const FDTDSolveOptions* o, FDTDSolveResult* res) {
         if (h->bc[a] != '0' && h->bc[a] != 'E' && h->bc[a] != 'H') periodic = true;
     bool small_index = (long long)h->Nz * h->Ny * ((h->Nx + 31) / 32 * 32) < (1LL << 31) &&
                        (long long)h->Nz * h->Ny * (h->w[0] + h->w[1]) < (1LL << 31);
-    // kernel ids: 0 auto, 1 scalar H/E pair, 3 fused z-marching step, 5
-    // vector H/E pair, 6 vector pair split into interior and rim launches.
-    // Auto takes the split pair in float32 when at least 60% of the warp
-    // tasks lie in no CPML slab (the 1201 x 601 x 301 grating slab, 69%:
-    // 3293 instead of 3605 us per step; the 321 x 161 x 101 MMI block, 23%:
-    // 143 instead of 122), else the vector pair.
+    // kernel ids: 0 auto, 1 scalar H/E pair, 3 fused step, 5 vector H/E pair, 6
+    // vector pair split into interior and rim launches.  Auto takes the fused
+    // step wherever it is possible but for rows of at most 16 vectors, which
+    // leave half of its lanes idle (64 x 64 x 64 in float32: 16.6 us per step
+    // against 14.6 for the vector pair; 72 x 72 x 72: 18.2 against 22.7; in
+    // float64, 64 x 64 x 64: 16.8 against 18.9).  Without it: the split pair in
+    // float32 when at least 60% of the warp tasks lie in no CPML slab (the
+    // 1201 x 601 x 301 grating slab, 69%: 3293 instead of 3605 us per step;
+    // the 321 x 161 x 101 MMI block, 23%: 143 instead of 122), else the
+    // vector pair.  All of them round alike, so the choice changes no bit.
+    bool split_rule = false;
+    if (sizeof(T) == 4 && !periodic && small_index)
+        split_rule = fdtdb::split_interior_fraction<T>(make_view<T>(h, r, 0)) >= 0.6;
     int kid = h->kernel;
-    if (kid == 0) {
-        kid = 5;
-        if (sizeof(T) == 4 && !periodic && small_index) {
-            const fdtdb::GridView<T> gv = make_view<T>(h, r, 0);
-            if (fdtdb::split_interior_fraction<T>(gv) >= 0.6) kid = 6;
-        }
+    const int pair = periodic || !small_index ? 1 : split_rule ? 6 : 5;
+    if (kid == 0) kid = march_possible<T>(h) && h->Nx > 16 * (16 / (int)sizeof(T)) ? 3 : pair;
+    else if (periodic || !small_index) kid = 1;
+    else if (kid == 3 && !march_possible<T>(h)) kid = pair;
+    int rc;
+    CK(cudaEventRecord(h->ev[2], h->stream));
+    rc = alloc_resident<T>(h, r, kid == 3);
+    if (rc != FDTD_OK && kid == 3 && h->kernel == 0) {
+        // no room for the second field set: the pair updates in place
+        cudaGetLastError();
+        r.release_all();
+        kid = pair;
+        rc = alloc_resident<T>(h, r, false);
     }
-    if (periodic || !small_index) kid = 1;
+    if (rc != FDTD_OK) return rc;
     const bool fused = kid == 3;
     const bool vec = kid == 5;
     const bool split = kid == 6;
-    int rc;
-    CK(cudaEventRecord(h->ev[2], h->stream));
-    if ((rc = alloc_resident<T>(h, r, fused)) != FDTD_OK) return rc;
     CK(cudaMemsetAsync(r.err.p, 0, sizeof(int) * 4, h->stream));
     if (!o->materials_unchanged || !r.coeffs_valid) {
         if ((rc = prepare_materials<T>(h, r)) != FDTD_OK) return rc;
@@ -1069,7 +1177,7 @@ int solve_impl(FDTDHandle* h, const FDTDSolveOptions* o, FDTDSolveResult* res) {
     for (int s = 0; s < (fused ? 2 : 1); s++) {
         for (int c = 0; c < 6; c++) CK(cudaMemsetAsync(r.F[s][c].p, 0, sizeof(T) * cells, h->stream));
         for (int a = 0; a < 3; a++)
-            for (int q = 0; q < 4; q++)
+            for (int q = 0; q < (s ? 2 : 4); q++)
                 CK(cudaMemsetAsync(r.psi[s][a][q].p, 0, r.psi[s][a][q].bytes, h->stream));
     }
     // convergence probe state
@@ -1099,7 +1207,11 @@ int solve_impl(FDTDHandle* h, const FDTDSolveOptions* o, FDTDSolveResult* res) {
 
     long long* sb = dptr<long long>(r.stepbase);
     fdtdb::GridView<T> g0 = make_view<T>(h, r, 0);
-    fdtdb::GridView<T> g1 = fused ? make_view<T>(h, r, 1) : g0;
+    fdtdb::MarchArgs<T> m0, m1;
+    if (fused) {
+        if ((rc = make_march<T>(h, r, 0, !split_rule, m0)) != FDTD_OK) return rc;
+        if ((rc = make_march<T>(h, r, 1, !split_rule, m1)) != FDTD_OK) return rc;
+    }
     T* f0[6];
     T* f1[6];
     for (int c = 0; c < 6; c++) {
@@ -1110,20 +1222,27 @@ int solve_impl(FDTDHandle* h, const FDTDSolveOptions* o, FDTDSolveResult* res) {
     auto cur_set = [&](long long steps) -> T* const* { return (fused && (steps & 1)) ? f1 : f0; };
     int dev_sms = 148;
     cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, h->device);
-    const int zc = h->zchunk > 0 ? h->zchunk : fdtdb::zmarch_chunk(h->Nx, h->Ny, h->Nz, dev_sms);
+    std::vector<int4> work;
+    if (fused) {
+        fdtdb::march_work<T>(g0, dev_sms, h->zchunk, work);
+        CK(r.work.ensure(sizeof(int4) * work.size()));
+        CK(cudaMemcpyAsync(r.work.p, work.data(), sizeof(int4) * work.size(), cudaMemcpyDefault, h->stream));
+        CK(cudaStreamSynchronize(h->stream));
+    }
+    // planes of the longest chunk, for the result
+    int zc = 0;
+    for (const int4& q : work) zc = std::max(zc, q.w - q.z);
     auto run = [&](long long n_first, long long count) -> int {
         fdtdb::launch_set_ll(sb, n_first, h->stream);
         launches += 1 + count * (fused ? 1 : 2);
         for (long long q = 0; q < count; q++) {
             const bool odd = (n_first + q) & 1;
             if (fused) {
-                CK(fdtdb::launch_step_zmarch<T>(odd ? g1 : g0, odd ? g0 : g1, odd ? f1 : f0,
-                                                odd ? f0 : f1, src, sb, (int)q, zc, h->stream));
+                CK(fdtdb::launch_step_march<T>(odd ? m1 : m0, src, dptr<int4>(r.work), (int)work.size(), sb, (int)q, h->stream));
             } else if (vec) {
                 CK(fdtdb::launch_step_vec<T>(g0, f0, src, sb, (int)q, h->stream));
             } else if (split) {
                 CK(fdtdb::launch_step_split<T>(g0, f0, src, sb, (int)q, h->stream));
-
             } else {
                 fdtdb::launch_step_unfused<T>(g0, f0, src, sb, (int)q, h->stream);
             }

@@ -103,7 +103,7 @@ __device__ __forceinline__ bool serve_running(int state) {
 
 // Local CPML slab index of coordinate c on axis a, or -1.
 template <typename T>
-__device__ __forceinline__ int slab_local(const PmlAxis<T>& P, int c, bool strict_max) {
+FDTD_HD int slab_local(const PmlAxis<T>& P, int c, bool strict_max) {
     if (c < P.w0) return c;
     if (strict_max ? (c > P.edge_max) : (c >= P.edge_max)) return P.w0 + (c - P.edge_max);
     return -1;

@@ -1,9 +1,13 @@
 // kernels.h -- host-side launch wrappers for the CUDA kernels.
 #pragma once
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <vector>
+
 #include "cell.cuh"
+#include "packed.cuh"
 
 namespace fdtdb {
 
@@ -36,18 +40,50 @@ cudaError_t launch_half_vec(const GridView<T>& g, T* const* fields, const Source
                             const long long* step_base, int off, int half, int i0, int ni,
                             cudaStream_t st);
 
-// One fused time step (zmarch_kernels.cu): H and E of every cell, reading the
-// fields and CPML state of (ga, fa) and writing those of (gb, fb); each
-// single-warp CTA marches a 60-cell row segment through zc planes.  Requires
-// non-periodic boundaries and a whole-grid view.
-template <typename T>
-cudaError_t launch_step_zmarch(const GridView<T>& ga, const GridView<T>& gb, T* const* fa,
-                               T* const* fb, const SourceList<T>& src, const long long* step_base,
-                               int off, int zc, cudaStream_t st);
+constexpr unsigned kMarchXBytes = 160;   // x-slab state of a row that one box copy brings
 
-// Planes per z chunk of the fused step: about 32 resident warps per SM on
-// `sms` multiprocessors, at least 4 planes.
-int zmarch_chunk(int Nx, int Ny, int Nz, int sms);
+// Arguments of the fused step (zmarch_kernels.cu): fields and H-update CPML
+// state are read from one set and written to the other; the E-update CPML
+// state is read and written by its own thread only, in place.  The x-slab
+// state has rows of x_pitch slots that start on 16 bytes: the min slab's
+// cells, rounded up to whole vectors, then the vectors from the one that
+// holds the first cell of the max slab (slot x_max_slot + k).  xtab: 1/kappa,
+// b, c of the H and the E update for every cell of a row (1, 0, 0 outside the
+// slabs).
+template <typename T>
+struct MarchArgs {
+    GridView<T> g;
+    Fields<T> in, out;
+    const T* ph_in[3][2];
+    T* ph_out[3][2];
+    T* pe[3][2];
+    const T* xtab[6];
+    // the same six values per local index of the y and z slabs, each in the
+    // form of a scalar argument
+    const typename pk::DupOf<T>::type *ytab, *ztab;
+    typename pk::DupOf<T>::type o[3], m[3], mone;   // R/d, uniform dt/mu, -1
+    // box copies: in, the E coefficients, the x-slab state (ph_in[0], pe[0])
+    CUtensorMap tm_in[6], tm_b[3], tm_x[4];
+    int* err;                        // set to 1 by a bounded wait that gives up
+    int x_pitch, x_max_slot, x_tiles;
+    int src_general;      // a 64-cell task that a source touches is not plain
+};
+
+// One fused time step: CTA k marches the tile (work[k].x, work[k].y) through
+// planes work[k].z .. work[k].w - 1.  Requires non-periodic boundaries, a
+// whole-grid view and 32-bit byte offsets.
+template <typename T>
+cudaError_t launch_step_march(const MarchArgs<T>& a, const SourceList<T>& src, const int4* work, int nwork,
+                              const long long* step_base, int off, cudaStream_t st);
+
+// Fills the tensor maps of `a` from its arrays.
+template <typename T>
+cudaError_t march_maps(MarchArgs<T>& a);
+
+// The work list of the fused step: chunks of zc planes, or (zc = 0) chunks of
+// equal estimated time for `sms` multiprocessors.
+template <typename T>
+void march_work(const GridView<T>& g, int sms, int zc, std::vector<int4>& work);
 
 // eps or mu (complex128, dense [Nz][Ny][Nx]) -> pitched update coefficients.
 // b = dt/eps.real, or for lossy media a = (er/dt - ei/2)/(er/dt + ei/2),

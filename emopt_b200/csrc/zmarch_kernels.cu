@@ -1,505 +1,722 @@
 // zmarch_kernels.cu -- one fused time step (H half step, then E half step)
-// per launch, each warp marching up a column of planes.
+// per launch, each CTA marching a tile of rows up through the planes.
 //
-// Arithmetic per cell: src/fdtd.cpp:175-310 (H) and :503-669 (E), in the same
-// association as the vector bodies (vec_body.cuh): curl scaled by R/d, CPML
-// corrections in x, y, z order with psi <- c d + b psi and (psi - d) + d/kappa,
-// sources after each half step, E beyond the max faces zero (PEC), the
-// symmetry rule at the min faces (src/fdtd.cpp:141-173, :397-501).
+// Arithmetic per cell: src/fdtd.cpp:175-310 (H) and :503-669 (E), with the
+// roundings of the vector pair (vec_body.cuh) written out as explicit
+// multiplies, adds and fused multiply-adds, so both give the same bits.
 //
-// Work of one warp (single-warp CTA): a 60-cell segment x0 .. x0+59 of row j,
-// for the planes i0 .. i1-1 of its z chunk.  Lane l holds the two cells
-// c0 = x0 - 2 + 2l, c0 + 1 (one float2 / double2 per array): lanes 1..30 own
-// the 60 cells; lane 0 computes H at x0 - 1 (the E update of cell x0 reads
-// it) and lane 31 only supplies E at x0 + 60 (the H update of x0 + 59 reads
-// it).  Per plane i the warp
-//   * loads E(i+1) of rows j-1, j and j+1, H(i) of rows j-1 and j and the E
-//     coefficients of row j -- E(i) of those rows and H(i-1) of row j are
-//     still in registers from the previous plane;
-//   * computes H(i) of row j and of row j-1 (the E update of row j reads Hx
-//     and Hz there; row j-1 belongs to another warp, which stores it);
-//   * computes E(i) of row j and stores H(i) and E(i) of row j.
-// The first plane of a chunk also recomputes H(i0-1) of row j.  Every value a
-// warp recomputes is read from the other field set, so the step reads set A
-// (fields and CPML state) and writes set B: no warp waits for another.
-// Each array is read from DRAM once per step; the halo rows and planes are L2
-// hits.  Bodies: M = 0 for warps whose cells, halo included, lie in no CPML
-// slab (no CPML code at all), M = -1 otherwise (run-time slab tests).
+// Work of one CTA: rows j0 .. j0+R-1 of one x tile for the planes i0 .. i1-1.
+// Warp w updates row j0 - 1 + w; a lane holds one 16-byte vector (4 float or
+// 2 double cells).  Warp 0 only recomputes H of row j0-1, lane 0 of a tile
+// (but the first) only H of the cells before it, lane 31 of a tile (but the
+// last) only supplies E, and the plane before the chunk is stepped for its H
+// alone: everything recomputed is read from the field set the step does not
+// write, so no CTA waits for another.  Each array crosses DRAM once per step.
+//
+// Data path: the tile's rows of E, H and the E coefficients come by TMA box
+// copies one to two planes ahead (rows, cells and planes outside the grid
+// arrive as zeros, the boundary value of E) into rings in shared memory; new
+// Hx, Hz go to the row above through shared memory.  One CTA barrier per plane
+// both publishes them and frees the ring slots the next copies overwrite.
+//
+// What bounds it: without CPML DRAM (321 x 161 x 101 cells in float32: 71 us a
+// step, 313 MB; 4.4 TB/s); with 20-cell slabs the latency of a plane, 4000
+// cycles for a CTA in no slab and 6500-9000 in one to three of them, of which
+// the slab state read from DRAM is the largest part.  16 warps per SM is what
+// 113 KB of shared memory and 128 registers leave, and any register spilled
+// inside the plane loop costs more than it saves (the L1 is all shared memory:
+// 16 bytes spilled took 193 us instead of 126).  us per step, before (vector
+// pair, in the large slab the interior/rim pair) and now, 15- or 20-cell slabs:
+//   float32  96x80x72 22.8 -> 18.7, 128x128x96 39.2 -> 31.0, 321x161x101
+//            122.8 -> 105.6, 801x401x201 1043 -> 920
+//   float64  101x76x65 27.0 -> 24.9, 321x161x101 207.5 -> 185
+#include <algorithm>
+#include <cmath>
+#include <queue>
+#include <utility>
+#include <vector>
+
 #include "kernels.h"
+#include "packed.cuh"
 #include "vec_body.cuh"
 
 namespace fdtdb {
 
 namespace {
 
-template <typename T>
-struct Pair {
-    T v[2];
-};
+__device__ __forceinline__ unsigned smem_u32(const void* p) {
+    return (unsigned)__cvta_generic_to_shared(p);
+}
 
+// The statements below touch shared memory and nothing else does; being
+// volatile they keep their order among themselves and against the barriers.
+__device__ __forceinline__ void mbar_init(unsigned bar) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar));
+}
+__device__ __forceinline__ void mbar_expect(unsigned bar, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes));
+}
+__device__ __forceinline__ bool mbar_try(unsigned bar, unsigned parity) {
+    unsigned done;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(done) : "r"(bar), "r"(parity));
+    return done != 0;
+}
+// Bounded wait for a copy group.  A wait that gives up reports through *err
+// (FDTD_solve_cw then fails) and returns true; the warp then runs on to its
+// end with single tries.
+__device__ __forceinline__ bool mbar_wait_slow(unsigned bar, unsigned parity, int* err, bool gave_up) {
+    for (int n = gave_up ? 0 : 1 << 16; n > 0; n--)
+        if (mbar_try(bar, parity)) return false;
+    atomicExch(err, 1);
+    return true;
+}
+__device__ __forceinline__ void l1_prefetch(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+// One vector in shared memory, at address a + OFF.
+template <typename T, unsigned OFF>
+__device__ __forceinline__ pk::Vec<T> sh_load(unsigned a) {
+    pk::Vec<T> r;
+    if constexpr (sizeof(T) == 4)
+        asm volatile("ld.shared.v2.b64 {%0, %1}, [%2+%3];" : "=l"(r.v[0]), "=l"(r.v[1]) : "r"(a), "n"(OFF));
+    else
+        asm volatile("ld.shared.v2.f64 {%0, %1}, [%2+%3];" : "=d"(r.v[0]), "=d"(r.v[1]) : "r"(a), "n"(OFF));
+    return r;
+}
+template <unsigned OFF>
+__device__ __forceinline__ void sh_store(unsigned a, const pk::Vec<float>& r) {
+    asm volatile("st.shared.v2.b64 [%0+%3], {%1, %2};" ::"r"(a), "l"(r.v[0]), "l"(r.v[1]), "n"(OFF));
+}
+template <unsigned OFF>
+__device__ __forceinline__ void sh_store(unsigned a, const pk::Vec<double>& r) {
+    asm volatile("st.shared.v2.f64 [%0+%3], {%1, %2};" ::"r"(a), "d"(r.v[0]), "d"(r.v[1]), "n"(OFF));
+}
+// Box copy of the rows y .. of plane z, cells x .. (x a multiple of 16 bytes).
+__device__ __forceinline__ void tma_box(unsigned dst, const CUtensorMap* map, int x, int y, int z, unsigned bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+        ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar));
+}
+
+// Global vectors, predicated without a branch, read once.
+__device__ __forceinline__ pk::Vec<float> gload(const float* p, unsigned ok) {
+    pk::Vec<float> r;
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n mov.b64 %0, 0;\n mov.b64 %1, 0;\n"
+        " @p ld.global.v2.b64 {%0, %1}, [%2];\n}"
+        : "=l"(r.v[0]), "=l"(r.v[1]) : "l"(p), "r"(ok));
+    return r;
+}
+__device__ __forceinline__ pk::Vec<double> gload(const double* p, unsigned ok) {
+    pk::Vec<double> r;
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n mov.f64 %0, 0d0000000000000000;\n mov.f64 %1, 0d0000000000000000;\n"
+        " @p ld.global.v2.f64 {%0, %1}, [%2];\n}"
+        : "=d"(r.v[0]), "=d"(r.v[1]) : "l"(p), "r"(ok));
+    return r;
+}
+__device__ __forceinline__ void gstore(float* p, const pk::Vec<float>& v, unsigned ok) {
+    asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n @p st.global.v2.b64 [%0], {%1, %2};\n}"
+                 ::"l"(p), "l"(v.v[0]), "l"(v.v[1]), "r"(ok));
+}
+__device__ __forceinline__ void gstore(double* p, const pk::Vec<double>& v, unsigned ok) {
+    asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n @p st.global.v2.f64 [%0], {%1, %2};\n}"
+                 ::"l"(p), "d"(v.v[0]), "d"(v.v[1]), "r"(ok));
+}
+// 1/kappa, b, c of one half step of a y or z slab entry (MarchArgs::ytab, ztab).
 template <typename T>
-__device__ __forceinline__ Pair<T> pload(const T* p, bool ok) {
-    Pair<T> r;
-    if (ok) {
-        // the read set is not written during the step: read-only cache path
-        typename vecb::V16<T>::type v = __ldg(reinterpret_cast<const typename vecb::V16<T>::type*>(p));
-        r.v[0] = v.x;
-        r.v[1] = v.y;
-    } else {
-        r.v[0] = T(0);
-        r.v[1] = T(0);
-    }
+struct Coef {
+    pk::Vec<T> k, b, c;
+};
+template <typename T>
+__device__ __forceinline__ Coef<T> coef(const typename pk::DupOf<T>::type* t) {
+    Coef<T> r;
+    r.k = pk::Vec<T>::dup(__ldg(t)); r.b = pk::Vec<T>::dup(__ldg(t + 1)); r.c = pk::Vec<T>::dup(__ldg(t + 2));
     return r;
 }
 
+// One array element block at a 32-bit byte offset: the base stays in uniform
+// registers, and all fields and coefficients share one offset register.
 template <typename T>
-__device__ __forceinline__ void pstore(T* p, T a, T b) {
-    typename vecb::V16<T>::type v;
-    v.x = a;
-    v.y = b;
-    *reinterpret_cast<typename vecb::V16<T>::type*>(p) = v;
+__device__ __forceinline__ const T* at(const T* base, unsigned off) {
+    return reinterpret_cast<const T*>(reinterpret_cast<const char*>(base) + off);
+}
+template <typename T>
+__device__ __forceinline__ T* at(T* base, unsigned off) {
+    return reinterpret_cast<T*>(reinterpret_cast<char*>(base) + off);
 }
 
-// CPML slots of one cell pair: x per cell (-1: none), y per row, z per plane.
-struct Slots {
-    int lx[2], ly, lz;
+// Shared memory, in bytes.  Ex and Ez sit in a ring of three planes (the tile's
+// rows, the row below and the row above); everything else in two stages that
+// alternate by plane: Ey, H (with the row below), the E coefficients, the new
+// Hx, Hz of the plane, the x-slab state (two accumulators of the H, two of
+// the E update, kXRow bytes a row).  Then the x-axis CPML tables, one vector
+// of zeros and the mbarriers.
+constexpr unsigned kRow = 512, kXRow = kMarchXBytes;
+template <int NW>
+struct MarchSmem {
+    static constexpr unsigned ring = 2 * (NW + 1) * kRow;            // one plane of Ex, Ez
+    static constexpr unsigned ez = (NW + 1) * kRow;                  // Ez within it
+    // within a stage
+    static constexpr unsigned ey = 0, h = ey + NW * kRow, b = h + 3 * NW * kRow, x = b + 3 * (NW - 1) * kRow,
+                              psx = x + 2 * NW * kRow, stage = (psx + 4 * NW * kXRow + 127) / 128 * 128;
+    static_assert(NW * kRow % 128 == 0 && NW * kXRow % 128 == 0, "box copies land on 128-byte boundaries");
+    static constexpr unsigned stage0 = 3 * ring, xt = stage0 + 2 * stage, zero = xt + 6 * kRow, bars = zero + 128;
+    static constexpr size_t bytes = bars + 64;
 };
 
-template <typename T, int M>
-__device__ __forceinline__ Slots slots_of(const GridView<T>& g, int i, int j, int c0, bool ok) {
-    Slots s;
-    s.ly = s.lz = -1;
-    s.lx[0] = s.lx[1] = -1;
-    if (M == 0 || !ok) return s;
-    s.ly = slab_local(g.pml[1], j, false);
-    s.lz = slab_local(g.pml[2], i + g.pml[2].off, true);
+__device__ __forceinline__ float sfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double sfma(double a, double b, double c) { return __fma_rn(a, b, c); }
+
+// Adds (magnetic, sign +) or subtracts (electric) the currents of the sources
+// in `mask` that drive this half step (base 3: M, 0: J) to one vector of cells,
+// in source order.  The coefficients of the next plane are brought to L1.
+template <typename T, int BASE>
+__device__ __forceinline__ void vec_sources(const SourceList<T>& src, unsigned mask, int i, int j, int c0, T S, T C,
+                                            pk::Vec<T>& a, pk::Vec<T>& b, pk::Vec<T>& c) {
+    constexpr int VW = pk::Vec<T>::N;
+    T f[3][VW];
+    a.get(f[0]); b.get(f[1]); c.get(f[2]);
+    for (; mask; mask &= mask - 1) {
+        const DevSource<T>& s = src.s[__ffs(mask) - 1];
+        const int li = i - s.i0, lj = j - s.j0;
 #pragma unroll
-    for (int e = 0; e < 2; e++) {
-        const int k = c0 + e;
-        s.lx[e] = (k >= 0 && k < g.Nx) ? slab_local(g.pml[0], k, false) : -1;
-    }
-    return s;
-}
-
-// psi of the H update (q = 0, 1) or the E update (q = 2, 3) of one cell
-// pair, all three axes: a[axis][q & 1][cell].
-template <typename T>
-struct Psi {
-    T a[3][2][2];
-};
-
-template <typename T, int M>
-__device__ __forceinline__ void psi_load(const GridView<T>& g, const Slots& s, int i, int j, int c0,
-                                         int q0, bool need0, bool need1, Psi<T>& p) {
-    if (M == 0) return;
-    const int Ny = g.Ny, px = g.px;
+        for (int e = 0; e < VW; e++) {
+            const int lk = c0 + e - s.k0;
+            if ((unsigned)lk >= (unsigned)s.K) continue;
+            const long long m = 2 * (((long long)li * s.J + lj) * s.K + lk);
 #pragma unroll
-    for (int e = 0; e < 2; e++)
-        if (s.lx[e] >= 0) {
-            const int o = (i * Ny + j) * g.pml[0].wsum + s.lx[e];
-            if (need0) p.a[0][0][e] = ld(g.pml[0].psi[q0] + o);
-            if (need1) p.a[0][1][e] = ld(g.pml[0].psi[q0 + 1] + o);
-        }
-    if (s.ly >= 0) {
-        const int o = (i * g.pml[1].wsum + s.ly) * px + c0;
-        if (need0) { Pair<T> t = pload<T>(g.pml[1].psi[q0] + o, true); p.a[1][0][0] = t.v[0]; p.a[1][0][1] = t.v[1]; }
-        if (need1) { Pair<T> t = pload<T>(g.pml[1].psi[q0 + 1] + o, true); p.a[1][1][0] = t.v[0]; p.a[1][1][1] = t.v[1]; }
-    }
-    if (s.lz >= 0) {
-        const int o = (s.lz * Ny + j) * px + c0;
-        if (need0) { Pair<T> t = pload<T>(g.pml[2].psi[q0] + o, true); p.a[2][0][0] = t.v[0]; p.a[2][0][1] = t.v[1]; }
-        if (need1) { Pair<T> t = pload<T>(g.pml[2].psi[q0 + 1] + o, true); p.a[2][1][0] = t.v[0]; p.a[2][1][1] = t.v[1]; }
-    }
-}
-
-template <typename T, int M>
-__device__ __forceinline__ void psi_store(const GridView<T>& g, const Slots& s, int i, int j, int c0,
-                                          int q0, const Psi<T>& p) {
-    if (M == 0) return;
-    const int Ny = g.Ny, px = g.px;
-#pragma unroll
-    for (int e = 0; e < 2; e++)
-        if (s.lx[e] >= 0) {
-            const int o = (i * Ny + j) * g.pml[0].wsum + s.lx[e];
-            g.pml[0].psi[q0][o] = p.a[0][0][e];
-            g.pml[0].psi[q0 + 1][o] = p.a[0][1][e];
-        }
-    if (s.ly >= 0) {
-        const int o = (i * g.pml[1].wsum + s.ly) * px + c0;
-        pstore<T>(g.pml[1].psi[q0] + o, p.a[1][0][0], p.a[1][0][1]);
-        pstore<T>(g.pml[1].psi[q0 + 1] + o, p.a[1][1][0], p.a[1][1][1]);
-    }
-    if (s.lz >= 0) {
-        const int o = (s.lz * Ny + j) * px + c0;
-        pstore<T>(g.pml[2].psi[q0] + o, p.a[2][0][0], p.a[2][0][1]);
-        pstore<T>(g.pml[2].psi[q0 + 1] + o, p.a[2][1][0], p.a[2][1][1]);
-    }
-}
-
-// E of one row of a plane: ex, ey, ez per cell of the pair.
-template <typename T>
-struct ERow {
-    T x[2], y[2], z[2];
-};
-
-// H of one cell pair: in the old values, out the new ones.  e: E of the row,
-// e_xn: Ey, Ez at c0 + 2 (first cell of the next lane), ejx/ejz: Ex, Ez of
-// row j+1, eix/eiy: Ex, Ey of plane i+1, mu: dt/mu per cell.  The CPML state
-// is updated in p (H slots).  Sources of row (i, j) are added when srcb.
-template <typename T, int M>
-__device__ __forceinline__ void h_pair(const GridView<T>& g, const SourceList<T>& src, int i, int j,
-                                       int c0, const ERow<T>& e, T ey_n, T ez_n, const T (&ejx)[2],
-                                       const T (&ejz)[2], const T (&eix)[2], const T (&eiy)[2],
-                                       const T (&mx)[2], const T (&my)[2], const T (&mz)[2],
-                                       const Slots& s, Psi<T>& p, bool srcb, T SH, T CH,
-                                       T (&hx)[2], T (&hy)[2], T (&hz)[2]) {
-#pragma unroll
-    for (int c = 0; c < 2; c++) {
-        const T eyx = c == 0 ? e.y[1] : ey_n;
-        const T ezx = c == 0 ? e.z[1] : ez_n;
-        const T dEzdy = g.ody * (ejz[c] - e.z[c]);
-        const T dEydz = g.odz * (eiy[c] - e.y[c]);
-        const T dExdz = g.odz * (eix[c] - e.x[c]);
-        const T dEzdx = g.odx * (ezx - e.z[c]);
-        const T dEydx = g.odx * (eyx - e.y[c]);
-        const T dExdy = g.ody * (ejx[c] - e.x[c]);
-        T Hx = hx[c] + mx[c] * (dEydz - dEzdy);
-        T Hy = hy[c] + my[c] * (dEzdx - dExdz);
-        T Hz = hz[c] + mz[c] * (dExdy - dEydx);
-        if (M != 0) {
-            if (s.lx[c] >= 0) {
-                const PmlAxis<T>& P = g.pml[0];
-                const int l = s.lx[c];
-                const T kv = ld(P.kinvH + l), bv = ld(P.bH + l), cv = ld(P.cH + l);
-                p.a[0][0][c] = cv * dEydx + bv * p.a[0][0][c];
-                p.a[0][1][c] = cv * dEzdx + bv * p.a[0][1][c];
-                Hz = Hz - mz[c] * ((p.a[0][0][c] - dEydx) + dEydx * kv);
-                Hy = Hy + my[c] * ((p.a[0][1][c] - dEzdx) + dEzdx * kv);
-            }
-            if (s.ly >= 0) {
-                const PmlAxis<T>& P = g.pml[1];
-                const T kv = ld(P.kinvH + s.ly), bv = ld(P.bH + s.ly), cv = ld(P.cH + s.ly);
-                p.a[1][0][c] = cv * dExdy + bv * p.a[1][0][c];
-                p.a[1][1][c] = cv * dEzdy + bv * p.a[1][1][c];
-                Hz = Hz + mz[c] * ((p.a[1][0][c] - dExdy) + dExdy * kv);
-                Hx = Hx - mx[c] * ((p.a[1][1][c] - dEzdy) + dEzdy * kv);
-            }
-            if (s.lz >= 0) {
-                const PmlAxis<T>& P = g.pml[2];
-                const T kv = ld(P.kinvH + s.lz), bv = ld(P.bH + s.lz), cv = ld(P.cH + s.lz);
-                p.a[2][0][c] = cv * dExdz + bv * p.a[2][0][c];
-                p.a[2][1][c] = cv * dEydz + bv * p.a[2][1][c];
-                Hx = Hx + mx[c] * ((p.a[2][1][c] - dEydz) + dEydz * kv);
-                Hy = Hy - my[c] * ((p.a[2][0][c] - dExdz) + dExdz * kv);
+            for (int q = 0; q < 3; q++) {
+                const T* p = s.comp[BASE + q];
+                if (!p) continue;
+                const T t = sfma(S, ld(p + m), C * ld(p + m + 1));
+                f[q][e] = BASE ? f[q][e] + t : f[q][e] - t;
+                if (li + 1 < s.I) asm volatile("prefetch.global.L1 [%0];" ::"l"(p + m + 2LL * s.J * s.K));
             }
         }
-        const int k = c0 + c;
-        if (srcb && k >= 0 && k < g.Nx) add_sources<T>(src, i, j, k, 3, SH, CH, Hx, Hy, Hz, false);
-        hx[c] = Hx; hy[c] = Hy; hz[c] = Hz;
     }
+    a.set(f[0]); b.set(f[1]); c.set(f[2]);
 }
 
-// dt/mu of a cell pair (uniform mu: the scalar of each component).
+// The curl terms oA fA - dB of a half step.  The vector pair's general body
+// rounds both products; its float32 body without CPML code (a plain cell)
+// fuses the first.  A warp's cells are all general (mode 0), all plain (1) or
+// mixed (2).  m: the rounded products dB on entry, the terms on return.
 template <typename T>
-__device__ __forceinline__ void mu_pair(const GridView<T>& g, int o, bool ok, T (&mx)[2], T (&my)[2],
-                                        T (&mz)[2]) {
-    if (g.bHarr[0] != nullptr) {
-        Pair<T> a = pload<T>(g.bHarr[0] + o, ok), b = pload<T>(g.bHarr[1] + o, ok),
-                c = pload<T>(g.bHarr[2] + o, ok);
+__device__ __forceinline__ void curls(int mode, bool plain, const pk::Vec<T> (&oA)[3], const pk::Vec<T> (&fA)[3],
+                                      pk::Vec<T> (&m)[3], const pk::Vec<T>& mone) {
+    if (sizeof(T) == 8 || mode == 0) {
 #pragma unroll
-        for (int e = 0; e < 2; e++) { mx[e] = a.v[e]; my[e] = b.v[e]; mz[e] = c.v[e]; }
+        for (int c = 0; c < 3; c++) m[c] = pk::diff(pk::mul(oA[c], fA[c]), m[c], mone);
+    } else if (mode == 1) {
+#pragma unroll
+        for (int c = 0; c < 3; c++) m[c] = pk::fma(oA[c], fA[c], pk::neg(m[c]));
     } else {
 #pragma unroll
-        for (int e = 0; e < 2; e++) { mx[e] = g.bH[0]; my[e] = g.bH[1]; mz[e] = g.bH[2]; }
+        for (int c = 0; c < 3; c++)
+            m[c] = pk::sel(plain, pk::fma(oA[c], fA[c], pk::neg(m[c])), pk::diff(pk::mul(oA[c], fA[c]), m[c], mone));
     }
 }
 
-template <typename T, int M>
-__device__ __forceinline__ void zm_body(const GridView<T>& ga, const GridView<T>& gb,
-                                        const Fields<T>& fa, const Fields<T>& fb,
-                                        const SourceList<T>& src, const long long* step_ctr,
-                                        int off, int x0, int j, int i0, int i1, int lane) {
-    constexpr unsigned FULL = 0xffffffffu;
-    const int Nx = ga.Nx, Ny = ga.Ny, Nz = ga.Nz, px = ga.px;
-    const int c0 = x0 - 2 + 2 * lane;
-    // a lane's pair is in the row when its first cell is (rows are padded to
-    // an even pitch, so the second cell never leaves the row's storage)
-    const bool ok = c0 >= 0 && c0 < Nx;
-    const bool own = ok && lane >= 1 && lane <= 30;
-    const bool hasj1 = j + 1 < Ny;
-    const bool hasjm = j > 0;
-    const long long plane = ga.plane;
-    const int rj = j * px + c0;   // offset of the pair within a plane
+// The value below a min face from the boundary rule (h_min_ghost of each cell).
+template <typename T>
+__device__ __forceinline__ pk::Vec<T> ghost(char bc, const pk::Vec<T>& first) {
+    if (bc == '0') return pk::Vec<T>::zero();
+    return bc == 'E' ? pk::neg(first) : first;
+}
 
-    // step constants of the sources
-    T SH = T(0), CH = T(0), SE = T(0), CE = T(0);
-    if (src.n) {
-        const double4 st = ga.step_tab[*step_ctr + off];
-        SH = T(st.x); CH = T(st.y); SE = T(st.z); CE = T(st.w);
-    }
-    // sources near this warp's cells in plane i, rows [ja, jb)
-    auto src_near = [&](int comp_base, int i, int ja, int jb) {
-        return src.n != 0 && vecb::sources_touch<T>(src, comp_base, i, ja, jb, x0 - 2, x0 + 62);
-    };
-
-    // E(i) of rows j-1, j, j+1 (the plane below the one the loop loads next)
-    ERow<T> em, e0;
-    T e1x[2], e1z[2];
-    auto load_erow = [&](ERow<T>& r, int i, int jj, bool row_ok) {
-        const bool q = ok && row_ok && i < Nz;
-        const long long o = (long long)i * plane + (long long)jj * px + c0;
-        Pair<T> a = pload<T>(fa.c[0] + o, q), b = pload<T>(fa.c[1] + o, q), c = pload<T>(fa.c[2] + o, q);
-        r.x[0] = a.v[0]; r.x[1] = a.v[1]; r.y[0] = b.v[0]; r.y[1] = b.v[1]; r.z[0] = c.v[0]; r.z[1] = c.v[1];
-    };
-    auto load_xz = [&](T (&x)[2], T (&z)[2], int i, int jj, bool row_ok) {
-        const bool q = ok && row_ok && i < Nz;
-        const long long o = (long long)i * plane + (long long)jj * px + c0;
-        Pair<T> a = pload<T>(fa.c[0] + o, q), c = pload<T>(fa.c[2] + o, q);
-        x[0] = a.v[0]; x[1] = a.v[1]; z[0] = c.v[0]; z[1] = c.v[1];
-    };
-    auto next_lane = [&](const ERow<T>& r, T& ey_n, T& ez_n) {
-        ey_n = __shfl_down_sync(FULL, r.y[0], 1);
-        ez_n = __shfl_down_sync(FULL, r.z[0], 1);
-    };
-
-    load_erow(e0, i0, j, true);
-    load_erow(em, i0, j - 1, hasjm);
-    load_xz(e1x, e1z, i0, j + 1, hasj1);
-
-    // H(i0 - 1) of row j: Hx and Hy, read by the E update of plane i0
-    T hpx[2], hpy[2];
-    if (i0 > 0) {
-        const int i = i0 - 1;
-        ERow<T> e;
-        T ejx[2], ejz[2], hx[2], hy[2], hz[2], mx[2], my[2], mz[2];
-        load_erow(e, i, j, true);
-        load_xz(ejx, ejz, i, j + 1, hasj1);
-        const long long o = (long long)i * plane + rj;
-        Pair<T> a = pload<T>(fa.c[3] + o, ok), b = pload<T>(fa.c[4] + o, ok);
-        hx[0] = a.v[0]; hx[1] = a.v[1]; hy[0] = b.v[0]; hy[1] = b.v[1]; hz[0] = hz[1] = T(0);
-        mu_pair<T>(ga, (int)o, ok, mx, my, mz);
-        const Slots s = slots_of<T, M>(ga, i, j, c0, ok);
-        Psi<T> p;
-        psi_load<T, M>(ga, s, i, j, c0, 0, true, true, p);
-        T ey_n, ez_n;
-        next_lane(e, ey_n, ez_n);
-        const T eix[2] = {e0.x[0], e0.x[1]}, eiy[2] = {e0.y[0], e0.y[1]};
-        h_pair<T, M>(ga, src, i, j, c0, e, ey_n, ez_n, ejx, ejz, eix, eiy, mx, my, mz, s, p,
-                     src_near(3, i, j, j + 1), SH, CH, hx, hy, hz);
-        hpx[0] = hx[0]; hpx[1] = hx[1]; hpy[0] = hy[0]; hpy[1] = hy[1];
-    } else {
-        hpx[0] = hpx[1] = hpy[0] = hpy[1] = T(0);
-    }
-
-    // CPML slots that do not change along the march: x per lane, y per row
-    Slots s_own = slots_of<T, M>(ga, 0, j, c0, ok);
-    Slots s_hal = slots_of<T, M>(ga, 0, j - 1, c0, ok && hasjm);
-
-    for (int i = i0; i < i1; i++) {
-        // ---- loads of the plane: E(i+1) of rows j-1, j, j+1, H(i) of rows
-        // j-1, j, the E coefficients, the CPML state of both rows
-        ERow<T> nm, n0;
-        T n1x[2], n1z[2];
-        load_erow(n0, i + 1, j, true);
-        load_erow(nm, i + 1, j - 1, hasjm);
-        load_xz(n1x, n1z, i + 1, j + 1, hasj1);
-        const long long o = (long long)i * plane + rj;
-        T hx[2], hy[2], hz[2], gx[2], gz[2];
-        {
-            Pair<T> a = pload<T>(fa.c[3] + o, ok), b = pload<T>(fa.c[4] + o, ok),
-                    c = pload<T>(fa.c[5] + o, ok);
-            hx[0] = a.v[0]; hx[1] = a.v[1]; hy[0] = b.v[0]; hy[1] = b.v[1]; hz[0] = c.v[0]; hz[1] = c.v[1];
-            Pair<T> d = pload<T>(fa.c[3] + o - px, ok && hasjm), f = pload<T>(fa.c[5] + o - px, ok && hasjm);
-            gx[0] = d.v[0]; gx[1] = d.v[1]; gz[0] = f.v[0]; gz[1] = f.v[1];
-        }
-        T bx[2], by[2], bz[2];
-        {
-            Pair<T> a = pload<T>(ga.bE[0] + o, ok), b = pload<T>(ga.bE[1] + o, ok),
-                    c = pload<T>(ga.bE[2] + o, ok);
-            bx[0] = a.v[0]; bx[1] = a.v[1]; by[0] = b.v[0]; by[1] = b.v[1]; bz[0] = c.v[0]; bz[1] = c.v[1];
-        }
-        Slots s = s_own, sm = s_hal;
-        if (M != 0) {
-            const int lz = slab_local(ga.pml[2], i + ga.pml[2].off, true);
-            s.lz = ok ? lz : -1;
-            sm.lz = ok && hasjm ? lz : -1;
-        }
-        Psi<T> ph, pe, pm;
-        psi_load<T, M>(ga, s, i, j, c0, 0, true, true, ph);
-        psi_load<T, M>(ga, s, i, j, c0, 2, true, true, pe);
-        psi_load<T, M>(ga, sm, i, j - 1, c0, 0, true, true, pm);
-        T mx[2], my[2], mz[2], gmx[2], gmy[2], gmz[2];
-        mu_pair<T>(ga, (int)o, ok, mx, my, mz);
-        mu_pair<T>(ga, (int)(o - px), ok && hasjm, gmx, gmy, gmz);
-
-        // ---- H(i) of row j, then of row j-1 (Hx, Hz only are used)
-        T ey_n, ez_n;
-        next_lane(e0, ey_n, ez_n);
-        {
-            const T eix[2] = {n0.x[0], n0.x[1]}, eiy[2] = {n0.y[0], n0.y[1]};
-            h_pair<T, M>(ga, src, i, j, c0, e0, ey_n, ez_n, e1x, e1z, eix, eiy, mx, my, mz, s, ph,
-                         src_near(3, i, j, j + 1), SH, CH, hx, hy, hz);
-        }
-        if (hasjm) {
-            T my_ey_n, my_ez_n;
-            next_lane(em, my_ey_n, my_ez_n);
-            const T ejx[2] = {e0.x[0], e0.x[1]}, ejz[2] = {e0.z[0], e0.z[1]};
-            const T eix[2] = {nm.x[0], nm.x[1]}, eiy[2] = {nm.y[0], nm.y[1]};
-            T gy[2] = {T(0), T(0)};
-            h_pair<T, M>(ga, src, i, j - 1, c0, em, my_ey_n, my_ez_n, ejx, ejz, eix, eiy, gmx, gmy,
-                         gmz, sm, pm, src_near(3, i, j - 1, j), SH, CH, gx, gy, gz);
-        }
-
-        // ---- E(i) of row j
-        // Hy, Hz at k - 1: the previous cell, across lanes by a shuffle
-        T hy_p = __shfl_up_sync(FULL, hy[1], 1), hz_p = __shfl_up_sync(FULL, hz[1], 1);
-        const bool lossy = ga.aE[0] != nullptr;
-        T ax[2], ay[2], az[2];
-        if (lossy) {
-            Pair<T> a = pload<T>(ga.aE[0] + o, ok), b = pload<T>(ga.aE[1] + o, ok), c = pload<T>(ga.aE[2] + o, ok);
-            ax[0] = a.v[0]; ax[1] = a.v[1]; ay[0] = b.v[0]; ay[1] = b.v[1]; az[0] = c.v[0]; az[1] = c.v[1];
-        }
-        const bool srce = src_near(0, i, j, j + 1);
-        T ex[2], ey[2], ez[2];
-#pragma unroll
-        for (int c = 0; c < 2; c++) {
-            const int k = c0 + c;
-            T hyx = c == 0 ? hy_p : hy[0];
-            T hzx = c == 0 ? hz_p : hz[0];
-            if (k == 0) { hyx = h_min_ghost<T>(ga.bc[0], hy[c], T(0)); hzx = h_min_ghost<T>(ga.bc[0], hz[c], T(0)); }
-            T hxj = gx[c], hzj = gz[c];
-            if (!hasjm) { hxj = h_min_ghost<T>(ga.bc[1], hx[c], T(0)); hzj = h_min_ghost<T>(ga.bc[1], hz[c], T(0)); }
-            T hxi = hpx[c], hyi = hpy[c];
-            if (i == 0) { hxi = h_min_ghost<T>(ga.bc[2], hx[c], T(0)); hyi = h_min_ghost<T>(ga.bc[2], hy[c], T(0)); }
-            const T dHzdy = ga.ody * (hz[c] - hzj);
-            const T dHydz = ga.odz * (hy[c] - hyi);
-            const T dHxdz = ga.odz * (hx[c] - hxi);
-            const T dHzdx = ga.odx * (hz[c] - hzx);
-            const T dHydx = ga.odx * (hy[c] - hyx);
-            const T dHxdy = ga.ody * (hx[c] - hxj);
-            T Ex, Ey, Ez;
-            if (lossy) {
-                Ex = ax[c] * e0.x[c] + (dHzdy - dHydz) * bx[c];
-                Ey = ay[c] * e0.y[c] + (dHxdz - dHzdx) * by[c];
-                Ez = az[c] * e0.z[c] + (dHydx - dHxdy) * bz[c];
-            } else {
-                Ex = e0.x[c] + (dHzdy - dHydz) * bx[c];
-                Ey = e0.y[c] + (dHxdz - dHzdx) * by[c];
-                Ez = e0.z[c] + (dHydx - dHxdy) * bz[c];
-            }
-            if (M != 0) {
-                if (s.lx[c] >= 0) {
-                    const PmlAxis<T>& P = ga.pml[0];
-                    const int l = s.lx[c];
-                    const T kv = ld(P.kinvE + l), bv = ld(P.bE + l), cv = ld(P.cE + l);
-                    pe.a[0][0][c] = cv * dHydx + bv * pe.a[0][0][c];
-                    pe.a[0][1][c] = cv * dHzdx + bv * pe.a[0][1][c];
-                    Ez = Ez + ((pe.a[0][0][c] - dHydx) + dHydx * kv) * bz[c];
-                    Ey = Ey - ((pe.a[0][1][c] - dHzdx) + dHzdx * kv) * by[c];
-                }
-                if (s.ly >= 0) {
-                    const PmlAxis<T>& P = ga.pml[1];
-                    const T kv = ld(P.kinvE + s.ly), bv = ld(P.bE + s.ly), cv = ld(P.cE + s.ly);
-                    pe.a[1][0][c] = cv * dHxdy + bv * pe.a[1][0][c];
-                    pe.a[1][1][c] = cv * dHzdy + bv * pe.a[1][1][c];
-                    Ez = Ez - ((pe.a[1][0][c] - dHxdy) + dHxdy * kv) * bz[c];
-                    Ex = Ex + ((pe.a[1][1][c] - dHzdy) + dHzdy * kv) * bx[c];
-                }
-                if (s.lz >= 0) {
-                    const PmlAxis<T>& P = ga.pml[2];
-                    const T kv = ld(P.kinvE + s.lz), bv = ld(P.bE + s.lz), cv = ld(P.cE + s.lz);
-                    pe.a[2][0][c] = cv * dHxdz + bv * pe.a[2][0][c];
-                    pe.a[2][1][c] = cv * dHydz + bv * pe.a[2][1][c];
-                    Ex = Ex - ((pe.a[2][1][c] - dHydz) + dHydz * kv) * bx[c];
-                    Ey = Ey + ((pe.a[2][0][c] - dHxdz) + dHxdz * kv) * by[c];
-                }
-            }
-            if (srce && k < Nx) add_sources<T>(src, i, j, k, 0, SE, CE, Ex, Ey, Ez, true);
-            ex[c] = Ex; ey[c] = Ey; ez[c] = Ez;
-        }
-
-        // ---- stores of row j (the 60 owned cells)
-        if (own) {
-            pstore<T>(fb.c[3] + o, hx[0], hx[1]);
-            pstore<T>(fb.c[4] + o, hy[0], hy[1]);
-            pstore<T>(fb.c[5] + o, hz[0], hz[1]);
-            pstore<T>(fb.c[0] + o, ex[0], ex[1]);
-            pstore<T>(fb.c[1] + o, ey[0], ey[1]);
-            pstore<T>(fb.c[2] + o, ez[0], ez[1]);
-            psi_store<T, M>(gb, s, i, j, c0, 0, ph);
-            psi_store<T, M>(gb, s, i, j, c0, 2, pe);
-        }
-
-        // ---- the next plane
-        hpx[0] = hx[0]; hpx[1] = hx[1]; hpy[0] = hy[0]; hpy[1] = hy[1];
-        e0 = n0;
-        em = nm;
-        e1x[0] = n1x[0]; e1x[1] = n1x[1]; e1z[0] = n1z[0]; e1z[1] = n1z[1];
-    }
+// psi <- c d + b psi, and the correction (psi - d) + d / kappa that is added
+// to the curl term d.
+template <typename T>
+__device__ __forceinline__ pk::Vec<T> cpml(pk::Vec<T>& p, const pk::Vec<T>& d, const pk::Vec<T>& kinv,
+                                           const pk::Vec<T>& b, const pk::Vec<T>& c, const pk::Vec<T>& mone) {
+    p = pk::fma(c, d, pk::mul(b, p));
+    return pk::fma(d, kinv, pk::diff(p, d, mone));
 }
 
 }  // namespace
 
-#ifndef ZM_MINB32
-#define ZM_MINB32 16
-#endif
-#define ZM_MINB(T) (sizeof(T) == 8 ? 0 : ZM_MINB32)
+template <typename T, int NW, int MINB, bool LOSSY, bool MUARR>
+__global__ void __launch_bounds__(32 * NW, MINB)
+k_step_march(const __grid_constant__ MarchArgs<T> A, const __grid_constant__ SourceList<T> src,
+             const int4* work, const long long* step_base, int off) {
+    using V = pk::Vec<T>;
+    using L = MarchSmem<NW>;
+    constexpr int VW = V::N, R = NW - 1;
+    constexpr unsigned SZ = sizeof(T);
+    extern __shared__ __align__(128) unsigned char smem[];
+    const GridView<T>& g = A.g;
+    const PmlAxis<T>& PX = g.pml[0];
+    const PmlAxis<T>& PY = g.pml[1];
+    const PmlAxis<T>& PZ = g.pml[2];
+    const int lane = threadIdx.x & 31, w = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+    const int4 job = __ldg(work + blockIdx.x);      // x tile, row tile, planes job.z .. job.w - 1
+    const int x0 = job.x * (30 * VW), c0 = x0 + lane * VW;
+    const int j0 = job.y * R, j = j0 - 1 + w;
+    const int i0 = job.z, i1 = job.w, is = i0 > 0 ? i0 - 1 : 0;
+    const bool row = j >= 0 && j < g.Ny;
+    const bool ok = row && c0 < g.Nx;
+    const bool own = ok && w > 0 && (lane > 0 || job.x == 0) && (lane < 31 || job.x == A.x_tiles - 1);
+    // byte offsets: a plane, this vector in a plane
+    const unsigned pb = (unsigned)g.Ny * g.px * SZ;
+    const unsigned rb = ok ? (unsigned)(j * g.px + c0) * SZ : 0u;
+    const unsigned sbase = smem_u32(smem), bars = sbase + L::bars;
+    const int ly = row ? slab_local(PY, j, false) : -1;
+    // x slab: slot of this vector in the whole-vector psi rows, or -1
+    int sx = -1;
+    if (c0 < PX.w0) sx = c0;
+    else if (c0 < g.Nx && c0 + VW > PX.edge_max && PX.w1 > 0) sx = A.x_max_slot + c0;
+    const bool inx = __any_sync(0xffffffffu, sx >= 0);
+    // the tile's slots, when they fit one box row, come by TMA as well
+    const int slo = __reduce_min_sync(0xffffffffu, sx >= 0 ? sx : 1 << 30), shi = __reduce_max_sync(0xffffffffu, sx);
+    const bool xtma = inx && (shi + VW - slo) * (int)SZ <= (int)kXRow;
+    const unsigned xoff = L::psx + w * kXRow + (unsigned)(sx >= 0 ? sx - slo : 0) * SZ;
+    if (!ok) sx = -1;
+    // float32: does the vector pair update this cell's 64-cell task by its
+    // body without CPML code in the planes of no z slab?
+    const int xb0 = c0 & ~63;
+    const bool plain = SZ == 4 && ly < 0 && xb0 >= PX.w0 && xb0 + 63 < PX.edge_max;
+    const int mode_xy = SZ == 8 ? 0
+                        : __all_sync(0xffffffffu, plain || !ok) ? 1
+                        : __any_sync(0xffffffffu, plain && ok)  ? 2
+                                                                : 0;
+    // sources whose box holds cells of this warp's row (bit q: M currents, 16 + q:
+    // J currents), and those that touch this cell's 64-cell task of the pair
+    unsigned touch = 0, task = 0;
+    if (row)
+        for (int q = 0; q < src.n; q++) {
+            const DevSource<T>& s = src.s[q];
+            if (j < s.j0 || j >= s.j0 + s.J) continue;
+            const unsigned bits = (s.comp[3] || s.comp[4] || s.comp[5] ? 1u << q : 0u) |
+                                  (s.comp[0] || s.comp[1] || s.comp[2] ? 0x10000u << q : 0u);
+            if (s.k0 < x0 + 32 * VW && s.k0 + s.K > x0) touch |= bits;
+            if (A.src_general && s.k0 < xb0 + 64 && s.k0 + s.K > xb0) task |= bits;
+        }
+    const unsigned near = __reduce_or_sync(0xffffffffu, touch | task);
+    T srcS[2] = {T(0), T(0)}, srcC[2] = {T(0), T(0)};     // step constants of the M and J currents
+    if (near) {
+        const double4 st = g.step_tab[*step_base + off];
+        srcS[0] = T(st.x); srcC[0] = T(st.y); srcS[1] = T(st.z); srcC[1] = T(st.w);
+    }
 
-// One time step: fields and CPML state read from (ga, fa), written to (gb, fb).
-// grid = (60-cell segments per row, rows, z chunks of zc planes); block = 32.
-template <typename T>
-__global__ void __launch_bounds__(32, ZM_MINB(T))
-k_step_zmarch(GridView<T> ga, GridView<T> gb, Fields<T> fa, Fields<T> fb, SourceList<T> src,
-              const long long* step_base, int off, int zc) {
-    const int x0 = blockIdx.x * 60;
-    const int j = blockIdx.y;
-    const int i0 = blockIdx.z * zc;
-    const int i1 = min(i0 + zc, ga.Nz);
-    // slab-free warp: cells x0-2 .. x0+61, rows j-1 .. j, planes i0-1 .. i1-1
-    const PmlAxis<T>& PX = ga.pml[0];
-    const PmlAxis<T>& PY = ga.pml[1];
-    const PmlAxis<T>& PZ = ga.pml[2];
-    const bool xin = x0 - 2 >= PX.w0 && x0 + 61 < PX.edge_max;
-    const bool yin = (j > 0 ? j - 1 : 0) >= PY.w0 && j < PY.edge_max;
-    const int zlo = (i0 > 0 ? i0 - 1 : 0) + PZ.off, zhi = i1 - 1 + PZ.off;
-    const bool zin = zlo >= PZ.w0 && (PZ.w1 == 0 || zhi <= PZ.edge_max);
-    if (xin && yin && zin)
-        zm_body<T, 0>(ga, gb, fa, fb, src, step_base, off, x0, j, i0, i1, threadIdx.x);
-    else
-        zm_body<T, -1>(ga, gb, fa, fb, src, step_base, off, x0, j, i0, i1, threadIdx.x);
+    bool gave_up = false;
+    auto wait = [&](unsigned bar, unsigned parity) {
+        if (!mbar_try(bar, parity)) gave_up = mbar_wait_slow(bar, parity, A.err, gave_up) || gave_up;
+    };
+    // Copies of one thread: E of plane p (Ez unless only read from below) into
+    // a ring slot; Ey of plane p and H of plane q into their stages; the
+    // coefficients of plane q.
+    const bool leader = threadIdx.x == 0;
+    auto stage_at = [&](int i) { return sbase + L::stage0 + (((i - is) & 1) ? L::stage : 0u); };
+    auto fetch_e = [&](int p, unsigned slot, bool full, unsigned bar) {
+        tma_box(slot, &A.tm_in[0], x0, j0 - 1, p, bar);
+        if (full) tma_box(slot + L::ez, &A.tm_in[2], x0, j0 - 1, p, bar);
+    };
+    auto fetch_x = [&](int q, int e, unsigned bar) {
+        if (!xtma) return;
+        const unsigned s = stage_at(q) + L::psx + 2 * e * NW * kXRow;
+        tma_box(s, &A.tm_x[2 * e], slo, j0 - 1, q, bar);
+        tma_box(s + NW * kXRow, &A.tm_x[2 * e + 1], slo, j0 - 1, q, bar);
+    };
+    auto fetch_eyh = [&](int p, int q, unsigned bar) {
+        tma_box(stage_at(p) + L::ey, &A.tm_in[1], x0, j0 - 1, p, bar);
+#pragma unroll
+        for (int c = 0; c < 3; c++)
+            tma_box(stage_at(q) + L::h + c * NW * kRow, &A.tm_in[3 + c], x0, j0 - 1, q, bar);
+        fetch_x(q, 0, bar);
+    };
+    const unsigned xbytes = xtma ? 2 * NW * kXRow : 0;
+    auto fetch_b = [&](int q, unsigned bar) {
+        mbar_expect(bar, 3 * (NW - 1) * kRow + xbytes);
+        fetch_x(q, 1, bar);
+#pragma unroll
+        for (int c = 0; c < 3; c++)
+            tma_box(stage_at(q) + L::b + c * (NW - 1) * kRow, &A.tm_b[c], x0, j0, q, bar);
+    };
+    const unsigned a_bytes = (2 * (NW + 1) + NW + 3 * NW) * kRow + xbytes;
+
+    // Per-thread addresses: E ring slots of planes i, i + 1, i + 2 (own row),
+    // stages of planes i and i + 1, and the barriers (A, then B 16 bytes on)
+    unsigned r0 = sbase, r1 = sbase + L::ring, r2 = sbase + 2 * L::ring;
+    unsigned sa = sbase + L::stage0, sb = sa + L::stage, ba = bars, bb = bars + 8;
+    if (leader) {
+        for (int q = 0; q < 4; q++) mbar_init(bars + 8 * q);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        // E(is), E(is+1), H(is) for the first plane; E(is+2), H(is+1) for the next
+        mbar_expect(ba, a_bytes + 2 * (NW + 1) * kRow - (is + 1 < i1 ? 0 : (NW + 1) * kRow));
+        fetch_e(is, r0, true, ba);
+        fetch_e(is + 1, r1, is + 1 < i1, ba);
+        fetch_eyh(is + 1, is, ba);
+        fetch_b(is, ba + 16);
+        if (is + 1 < i1) {
+            mbar_expect(bb, a_bytes - (is + 2 < i1 ? 0 : (NW + 1) * kRow));
+            fetch_e(is + 2, r2, is + 2 < i1, bb);
+            fetch_eyh(is + 2, is + 1, bb);
+        }
+    }
+    static_assert(NW == 8, "the copies are spread over eight warps");
+    const unsigned lrow = w * kRow + lane * 16;
+    r0 += lrow; r1 += lrow; r2 += lrow; sa += lrow; sb += lrow;
+    if (w == NW - 1)
+        for (int q = 0; q < 6; q++)
+            sh_store<0>(sbase + L::xt + q * kRow + lane * 16, V::load(A.xtab[q] + (c0 < g.px ? c0 : 0)));
+    if (threadIdx.x == 32) sh_store<0>(sbase + L::zero, V::zero());
+    const unsigned xta = sbase + L::xt + lane * 16;
+    V ey = V::zero(), hpy = V::zero();      // Ey of the plane, new Hy of the plane below
+    if (ok) ey = V::load(at(A.in.c[1], (unsigned)is * pb + rb));
+    __syncthreads();
+
+    const bool iny = ly >= 0, xmin = job.x == 0;
+    unsigned o = (unsigned)is * pb + rb;                              // this vector in the fields,
+    unsigned oX = ((unsigned)(is * g.Ny + j) * A.x_pitch + sx) * SZ;  // in the x- and y-slab state
+    unsigned oY = ((unsigned)(is * PY.wsum + ly) * g.px + (ok ? c0 : 0)) * SZ;
+    const unsigned strideY = (unsigned)PY.wsum * g.px * SZ, strideX = (unsigned)g.Ny * A.x_pitch * SZ;
+    const unsigned sxu = sx >= 0, ownu = own, ownxu = own && sx >= 0;
+    // x-slab state in a stage relative to sa (lanes without a slot read zeros)
+    const unsigned xz = sbase + L::zero;
+    const V ox = V::dup(A.o[0]), oy = V::dup(A.o[1]), oz = V::dup(A.o[2]), mone = V::dup(A.mone);
+    unsigned phase = 0;
+
+#pragma unroll 1
+    for (int i = is; i < i1; i++) {
+        const int lz = slab_local(PZ, i + PZ.off, true);
+        const bool inz = lz >= 0, emit = i >= i0;      // the plane before the chunk: H only
+        const unsigned oZ = (unsigned)lz * pb + rb;
+        const unsigned eo = emit ? ownu : 0u, eox = emit ? ownxu : 0u;
+
+        // ---- CPML state of the H update
+        V py0, py1, pz0, pz1;
+        if (iny) { py0 = gload(at(A.ph_in[1][0], oY), 1u); py1 = gload(at(A.ph_in[1][1], oY), 1u); }
+        if (inz) { pz0 = gload(at(A.ph_in[2][0], oZ), 1u); pz1 = gload(at(A.ph_in[2][1], oZ), 1u); }
+
+        // ---- which cells round their curls as the vector pair's plain body;
+        // the sources of this row in this plane
+        int modeH = inz ? 0 : mode_xy, modeE = modeH;
+        bool plH = plain, plE = plain;
+        unsigned now = 0;
+        if (near) {
+            for (int q = 0; q < src.n; q++)
+                if (i >= src.s[q].i0 && i < src.s[q].i0 + src.s[q].I) now |= 0x10001u << q;
+            now &= near;
+            if (modeH && A.src_general && now) {
+                // a task that a source touches takes the general body
+                plH = plain && !(task & now & 0xffffu);
+                plE = plain && !(task & now & 0xffff0000u);
+                modeH = modeE = 2;
+            }
+            now &= touch;
+        }
+
+        // ---- E of the plane, the row above and the plane above; H
+        wait(ba, phase);
+        if (i + 1 < i1) {
+            if (iny) { l1_prefetch(at(A.ph_in[1][0], oY + strideY)); l1_prefetch(at(A.ph_in[1][1], oY + strideY)); }
+            if (inz) { l1_prefetch(at(A.ph_in[2][0], oZ + pb)); l1_prefetch(at(A.ph_in[2][1], oZ + pb)); }
+        }
+        V ex = sh_load<T, 0>(r0), ez = sh_load<T, L::ez>(r0);
+        const V exj = sh_load<T, kRow>(r0), ezj = sh_load<T, L::ez + kRow>(r0);
+        const V exi = sh_load<T, 0>(r1), eyi = sh_load<T, L::ey>(sb);
+        V hx = sh_load<T, L::h>(sa), hy = sh_load<T, L::h + NW * kRow>(sa), hz = sh_load<T, L::h + 2 * NW * kRow>(sa);
+
+        // ---- H update
+        {
+            const V fzdy = pk::sub(ezj, ez), fydz = pk::sub(eyi, ey), fxdz = pk::sub(exi, ex);
+            const V fzdx = ez.diff_down(), fydx = ey.diff_down(), fxdy = pk::sub(exj, ex);
+            V m0, m1, m2;
+            if (MUARR) {
+                m0 = gload(at(g.bHarr[0], o), ok ? 1u : 0u); m1 = gload(at(g.bHarr[1], o), ok ? 1u : 0u);
+                m2 = gload(at(g.bHarr[2], o), ok ? 1u : 0u);
+            } else {
+                m0 = V::dup(A.m[0]); m1 = V::dup(A.m[1]); m2 = V::dup(A.m[2]);
+            }
+            const V oA[3] = {oz, ox, oy}, fA[3] = {fydz, fzdx, fxdy};
+            V t[3] = {pk::mul(oy, fzdy), pk::mul(oz, fxdz), pk::mul(ox, fydx)};
+            curls<T>(modeH, plH, oA, fA, t, mone);
+            hx = pk::fma(m0, t[0], hx);
+            hy = pk::fma(m1, t[1], hy);
+            hz = pk::fma(m2, t[2], hz);
+            if (inx) {
+                const V kv = sh_load<T, 0>(xta), bv = sh_load<T, kRow>(xta), cv = sh_load<T, 2 * kRow>(xta);
+                V p0, p1;
+                if (xtma) {
+                    const unsigned q = sxu ? sa - lrow + xoff : xz;
+                    p0 = sh_load<T, 0>(q);
+                    p1 = sh_load<T, 0>(sxu ? q + NW * kXRow : q);
+                } else {
+                    p0 = gload(at(A.ph_in[0][0], oX), sxu); p1 = gload(at(A.ph_in[0][1], oX), sxu);
+                }
+                hz = pk::fnma(m2, cpml(p0, pk::mul(ox, fydx), kv, bv, cv, mone), hz);
+                hy = pk::fma(m1, cpml(p1, pk::mul(ox, fzdx), kv, bv, cv, mone), hy);
+                gstore(at(A.ph_out[0][0], oX), p0, eox); gstore(at(A.ph_out[0][1], oX), p1, eox);
+            }
+            if (iny) {
+                const Coef<T> c = coef<T>(A.ytab + 6 * ly);
+                hz = pk::fma(m2, cpml(py0, pk::mul(oy, fxdy), c.k, c.b, c.c, mone), hz);
+                hx = pk::fnma(m0, cpml(py1, pk::mul(oy, fzdy), c.k, c.b, c.c, mone), hx);
+                gstore(at(A.ph_out[1][0], oY), py0, eo); gstore(at(A.ph_out[1][1], oY), py1, eo);
+            }
+            if (inz) {
+                const Coef<T> c = coef<T>(A.ztab + 6 * lz);
+                hx = pk::fma(m0, cpml(pz1, pk::mul(oz, fydz), c.k, c.b, c.c, mone), hx);
+                hy = pk::fnma(m1, cpml(pz0, pk::mul(oz, fxdz), c.k, c.b, c.c, mone), hy);
+                gstore(at(A.ph_out[2][0], oZ), pz0, eo); gstore(at(A.ph_out[2][1], oZ), pz1, eo);
+            }
+        }
+        if (now & 0xffffu) vec_sources<T, 3>(src, now & 0xffffu, i, j, c0, srcS[0], srcC[0], hx, hy, hz);
+        sh_store<L::x>(sa, hx);
+        sh_store<L::x + NW * kRow>(sa, hz);
+        gstore(at(A.out.c[3], o), hx, eo);
+        gstore(at(A.out.c[4], o), hy, eo);
+        gstore(at(A.out.c[5], o), hz, eo);
+
+        // ---- CPML state of the E update
+        if (iny) { py0 = gload(at(A.pe[1][0], oY), eo); py1 = gload(at(A.pe[1][1], oY), eo); }
+        if (inz) { pz0 = gload(at(A.pe[2][0], oZ), eo); pz1 = gload(at(A.pe[2][1], oZ), eo); }
+        __syncthreads();
+        // E(i), Ey(i+1), H(i) and the coefficients of plane i - 1 have been read:
+        // the next copies, spread over the warps (one issue takes ~200 cycles)
+        if (lane == 0) {
+            int v = w;
+            asm volatile("" : "+r"(v));              // keeps what follows out of registers between planes
+            if (v == 0) {
+                if (i + 2 < i1) {
+                    const bool full = i + 3 < i1;
+                    mbar_expect(ba, a_bytes - (full ? 0 : (NW + 1) * kRow));
+                    fetch_e(i + 3, r0, full, ba);
+                    fetch_x(i + 2, 0, ba);
+                }
+                if (i + 1 < i1) {
+                    mbar_expect(bb + 16, 3 * (NW - 1) * kRow + xbytes);
+                    fetch_x(i + 1, 1, bb + 16);
+                }
+            } else if (v < 5) {
+                // Ey of plane i + 3 (warp 1), H of plane i + 2 (2..4)
+                if (i + 2 < i1)
+                    tma_box((v == 1 ? sb + L::ey : sa + L::h + (v - 2) * NW * kRow) - v * kRow, &A.tm_in[v == 1 ? 1 : v + 1],
+                            x0, j0 - 1, v == 1 ? i + 3 : i + 2, ba);
+            } else if (i + 1 < i1) {
+                // the coefficients of plane i + 1
+                tma_box(sb + L::b + (v - 5) * (NW - 1) * kRow - v * kRow, &A.tm_b[v - 5], x0, j0, i + 1, bb + 16);
+            }
+        }
+        if (w > 0) {
+            wait(ba + 16, phase);
+            if (emit) {
+                const V bx = sh_load<T, L::b - kRow>(sa), by = sh_load<T, L::b + (NW - 2) * kRow>(sa),
+                        bz = sh_load<T, L::b + (2 * NW - 3) * kRow>(sa);
+                V hxj = sh_load<T, L::x - kRow>(sa), hzj = sh_load<T, L::x + (NW - 1) * kRow>(sa);   // the row below's
+                V hpx = sh_load<T, L::x>(sb);                                                       // the plane below's
+                if (j == 0) {
+                    hxj = ghost<T>(g.bc[1], hx);
+                    hzj = ghost<T>(g.bc[1], hz);
+                }
+                if (i == 0) { hpx = ghost<T>(g.bc[2], hx); hpy = ghost<T>(g.bc[2], hy); }
+                const V fzdy = pk::sub(hz, hzj), fydz = pk::sub(hy, hpy), fxdz = pk::sub(hx, hpx), fxdy = pk::sub(hx, hxj);
+                // differences to the cells k - 1
+                const bool first = xmin && c0 == 0;
+                const V fzdx = hz.diff_up(first, first ? h_min_ghost<T>(g.bc[0], hz.at0(), T(0)) : T(0));
+                const V fydx = hy.diff_up(first, first ? h_min_ghost<T>(g.bc[0], hy.at0(), T(0)) : T(0));
+                const V oA[3] = {oy, oz, ox}, fA[3] = {fzdy, fxdz, fydx};
+                V t[3] = {pk::mul(oz, fydz), pk::mul(ox, fzdx), pk::mul(oy, fxdy)};
+                curls<T>(modeE, plE, oA, fA, t, mone);
+                if (LOSSY) {
+                    ex = pk::fma(gload(at(g.aE[0], o), ownu), ex, pk::mul(t[0], bx));
+                    ey = pk::fma(gload(at(g.aE[1], o), ownu), ey, pk::mul(t[1], by));
+                    ez = pk::fma(gload(at(g.aE[2], o), ownu), ez, pk::mul(t[2], bz));
+                } else {
+                    ex = pk::fma(t[0], bx, ex); ey = pk::fma(t[1], by, ey); ez = pk::fma(t[2], bz, ez);
+                }
+                if (inx) {
+                    const V kv = sh_load<T, 3 * kRow>(xta), bv = sh_load<T, 4 * kRow>(xta), cv = sh_load<T, 5 * kRow>(xta);
+                    V p0, p1;
+                    if (xtma) {
+                        const unsigned q = sxu ? sa - lrow + xoff + 2 * NW * kXRow : xz;
+                        p0 = sh_load<T, 0>(q);
+                        p1 = sh_load<T, 0>(sxu ? q + NW * kXRow : q);
+                    } else {
+                        p0 = gload(at(A.pe[0][0], oX), ownxu); p1 = gload(at(A.pe[0][1], oX), ownxu);
+                    }
+                    ez = pk::fma(cpml(p0, pk::mul(ox, fydx), kv, bv, cv, mone), bz, ez);
+                    ey = pk::fnma(cpml(p1, pk::mul(ox, fzdx), kv, bv, cv, mone), by, ey);
+                    gstore(at(A.pe[0][0], oX), p0, ownxu); gstore(at(A.pe[0][1], oX), p1, ownxu);
+                }
+                if (iny) {
+                    const Coef<T> c = coef<T>(A.ytab + 6 * ly + 3);
+                    ez = pk::fnma(cpml(py0, pk::mul(oy, fxdy), c.k, c.b, c.c, mone), bz, ez);
+                    ex = pk::fma(cpml(py1, pk::mul(oy, fzdy), c.k, c.b, c.c, mone), bx, ex);
+                    gstore(at(A.pe[1][0], oY), py0, ownu); gstore(at(A.pe[1][1], oY), py1, ownu);
+                }
+                if (inz) {
+                    const Coef<T> c = coef<T>(A.ztab + 6 * lz + 3);
+                    ex = pk::fnma(cpml(pz1, pk::mul(oz, fydz), c.k, c.b, c.c, mone), bx, ex);
+                    ey = pk::fma(cpml(pz0, pk::mul(oz, fxdz), c.k, c.b, c.c, mone), by, ey);
+                    gstore(at(A.pe[2][0], oZ), pz0, ownu); gstore(at(A.pe[2][1], oZ), pz1, ownu);
+                }
+                if (now >> 16) vec_sources<T, 0>(src, now >> 16, i, j, c0, srcS[1], srcC[1], ex, ey, ez);
+                gstore(at(A.out.c[0], o), ex, ownu);
+                gstore(at(A.out.c[1], o), ey, ownu);
+                gstore(at(A.out.c[2], o), ez, ownu);
+            }
+        }
+        ey = eyi;
+        hpy = hy;
+        unsigned q = r0;
+        r0 = r1; r1 = r2; r2 = q;
+        q = sa; sa = sb; sb = q;
+        phase ^= (unsigned)(i - is) & 1u;
+        q = ba; ba = bb; bb = q;
+        o += pb; oX += strideX; oY += strideY;
+    }
+    // after a wait that gave up, time for copies still in flight to land
+    if (gave_up)
+        for (int n = 0; n < 4096; n++) __nanosleep(1000);
 }
 
-template <typename T>
-cudaError_t launch_step_zmarch(const GridView<T>& ga, const GridView<T>& gb, T* const* fa,
-                               T* const* fb, const SourceList<T>& src, const long long* step_base,
-                               int off, int zc, cudaStream_t st) {
-    Fields<T> a, b;
-    for (int c = 0; c < 6; c++) { a.c[c] = fa[c]; b.c[c] = fb[c]; }
-    if (zc <= 0) zc = ga.Nz;
-    dim3 grid((ga.Nx + 59) / 60, ga.Ny, (ga.Nz + zc - 1) / zc);
-    k_step_zmarch<T><<<grid, 32, 0, st>>>(ga, gb, a, b, src, step_base, off, zc);
+namespace {
+
+// Rows per CTA plus one: 8 warps, 2 CTAs (16 warps) per SM.
+constexpr int kNW = 8, kMinB = 2;
+
+template <typename T, bool LOSSY, bool MUARR>
+cudaError_t launch_one(const MarchArgs<T>& a, const SourceList<T>& src, const int4* work, int nwork,
+                       const long long* step_base, int off, cudaStream_t st) {
+    constexpr size_t bytes = MarchSmem<kNW>::bytes;
+    auto k = k_step_march<T, kNW, kMinB, LOSSY, MUARR>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) return e;
+    k<<<nwork, 32 * kNW, bytes, st>>>(a, src, work, step_base, off);
     return cudaGetLastError();
 }
 
-int zmarch_chunk(int Nx, int Ny, int Nz, int sms) {
-    // enough single-warp CTAs for about 32 per SM, chunks of at least 4 planes
-    const long long cols = (long long)((Nx + 59) / 60) * Ny;
-    const long long want = 32LL * (sms > 0 ? sms : 148);
-    int nchunk = (int)((want + cols - 1) / cols);
-    if (nchunk < 1) nchunk = 1;
-    int zc = (Nz + nchunk - 1) / nchunk;
-    if (zc < 4) zc = 4;
-    if (zc > Nz) zc = Nz;
-    return zc;
+template <typename T>
+int x_tiles(int Nx) {
+    constexpr int V = pk::Vec<T>::N;
+    return std::max(1, (Nx - 2 * V + 30 * V - 1) / (30 * V));
 }
 
-template cudaError_t launch_step_zmarch<float>(const GridView<float>&, const GridView<float>&,
-                                               float* const*, float* const*,
-                                               const SourceList<float>&, const long long*, int, int,
-                                               cudaStream_t);
-template cudaError_t launch_step_zmarch<double>(const GridView<double>&, const GridView<double>&,
-                                                double* const*, double* const*,
-                                                const SourceList<double>&, const long long*, int,
-                                                int, cudaStream_t);
+}  // namespace
+
+template <typename T>
+cudaError_t march_maps(MarchArgs<T>& a) {
+    using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult st;
+    cudaError_t e = cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &st);
+    if (e != cudaSuccess) return e;
+    if (st != cudaDriverEntryPointSuccess || !fn) return cudaErrorNotSupported;
+    const GridView<T>& g = a.g;
+    a.x_tiles = x_tiles<T>(g.Nx);
+    const CUtensorMapDataType type = sizeof(T) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64;
+    auto map = [&](CUtensorMap* m, const T* p, int rows) {
+        const cuuint64_t dims[3] = {(cuuint64_t)g.Nx, (cuuint64_t)g.Ny, (cuuint64_t)g.Nz};
+        const cuuint64_t strides[2] = {(cuuint64_t)g.px * sizeof(T), (cuuint64_t)g.plane * sizeof(T)};
+        const cuuint32_t box[3] = {(cuuint32_t)(512 / sizeof(T)), (cuuint32_t)rows, 1}, one[3] = {1, 1, 1};
+        return ((Encode)fn)(m, type, 3, const_cast<T*>(p), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    };
+    CUresult r = CUDA_SUCCESS;
+    for (int c = 0; c < 6 && r == CUDA_SUCCESS; c++)
+        r = map(&a.tm_in[c], a.in.c[c], c == 0 || c == 2 ? kNW + 1 : kNW);   // Ex, Ez: the row above too
+    for (int c = 0; c < 3 && r == CUDA_SUCCESS; c++) r = map(&a.tm_b[c], g.bE[c], kNW - 1);
+    for (int c = 0; c < 4 && a.x_pitch > 0 && r == CUDA_SUCCESS; c++) {
+        const cuuint64_t dims[3] = {(cuuint64_t)a.x_pitch, (cuuint64_t)g.Ny, (cuuint64_t)g.Nz};
+        const cuuint64_t strides[2] = {(cuuint64_t)a.x_pitch * sizeof(T), (cuuint64_t)a.x_pitch * g.Ny * sizeof(T)};
+        const cuuint32_t box[3] = {(cuuint32_t)(kMarchXBytes / sizeof(T)), kNW, 1}, one[3] = {1, 1, 1};
+        r = ((Encode)fn)(&a.tm_x[c], type, 3, c < 2 ? const_cast<T*>(a.ph_in[0][c]) : a.pe[0][c - 2], dims, strides,
+                         box, one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                         CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    }
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
+template <typename T>
+cudaError_t launch_step_march(const MarchArgs<T>& a, const SourceList<T>& src, const int4* work, int nwork,
+                              const long long* step_base, int off, cudaStream_t st) {
+    const bool lossy = a.g.aE[0] != nullptr, mu = a.g.bHarr[0] != nullptr;
+    if (lossy) return mu ? launch_one<T, true, true>(a, src, work, nwork, step_base, off, st)
+                         : launch_one<T, true, false>(a, src, work, nwork, step_base, off, st);
+    return mu ? launch_one<T, false, true>(a, src, work, nwork, step_base, off, st)
+              : launch_one<T, false, false>(a, src, work, nwork, step_base, off, st);
+}
+
+// The chunks of the tile columns.  A CTA takes as long as its slowest warp, and
+// CPML state makes planes slow (cycles per plane on the 321 x 161 x 101 grid
+// with 20-cell slabs: 3650 in none, 4600 in an x slab, 5900 z, 6700 y, 8300 in
+// all three), so every column is cut into chunks of equal estimated time, the
+// column with the longest ones first.  Chunks of 8 planes on average, in as many
+// waves as that takes, keep neighbouring tiles close in z (their halo rows hit
+// L2) and the last wave short: 105.6 us a step on that grid against 107.5 with
+// 9-13 planes, 118 in one wave and 125.6 in equal chunks of 26; in float64 185
+// against 227 in one wave.  Grids that fill less than a wave take one wave.
+template <typename T>
+void march_work(const GridView<T>& g, int sms, int zc, std::vector<int4>& work) {
+    constexpr int V = pk::Vec<T>::N, R = kNW - 1;
+    const int ntx = x_tiles<T>(g.Nx), nty = (g.Ny + R - 1) / R, Nz = g.Nz;
+    work.clear();
+    if (zc > 0) {
+        for (int i = 0; i < Nz; i += zc)
+            for (int y = 0; y < nty; y++)
+                for (int x = 0; x < ntx; x++) work.push_back(make_int4(x, y, i, std::min(i + zc, Nz)));
+        return;
+    }
+    const PmlAxis<T>*P = g.pml;
+    std::vector<char> inz(Nz);
+    int nz_slab = 0;
+    for (int i = 0; i < Nz; i++) nz_slab += inz[i] = slab_local(P[2], i + P[2].off, true) >= 0;
+    // estimated cycles (thousands) of a plane of column (x, y), outside and in a z slab
+    auto cost = [&](int x, int y, bool z) {
+        const int c0 = x * 30 * V, c1 = std::min(c0 + 32 * V, g.Nx), j0 = std::max(0, y * R - 1), j1 = std::min(y * R + R, g.Ny);
+        const bool sx = c0 < P[0].w0 || (P[0].w1 > 0 && c1 > P[0].edge_max);
+        const bool sy = j0 < P[1].w0 || (P[1].w1 > 0 && j1 > P[1].edge_max);
+        return 3.65 + (sx ? 0.9 : 0.0) + (sy && z ? 3.8 : sy ? 3.0 : z ? 2.2 : 0.0);
+    };
+    const int ncol = ntx * nty, slots = std::max(1, kMinB * (sms > 0 ? sms : 148));
+    const double fill = 8.0;                       // first copies and the plane before the chunk
+    std::vector<double> total(ncol);
+    for (int c = 0; c < ncol; c++)
+        total[c] = nz_slab * cost(c % ntx, c / ntx, true) + (Nz - nz_slab) * cost(c % ntx, c / ntx, false);
+    // kChunk planes a chunk on average, one wave of CTAs at least; the column with
+    // the longest chunks is cut first
+    constexpr double kChunk = 8.0;
+    const int waves = std::max(1, (int)std::lround((double)ncol * Nz / (kChunk * slots)));
+    std::vector<int> best(ncol, 1);
+    std::priority_queue<std::pair<double, int>> longest;
+    for (int c = 0; c < ncol; c++) longest.push({total[c] + fill, c});
+    for (long long k = ncol; k < (long long)waves * slots; k++) {
+        const int c = longest.top().second;
+        if (best[c] >= Nz) break;
+        longest.pop();
+        best[c]++;
+        longest.push({total[c] / best[c] + fill, c});
+    }
+    // cut the columns; chunk k of every column before chunk k + 1 of any
+    std::vector<std::vector<int4>> rank;
+    for (int c = 0; c < ncol; c++) {
+        const double in = cost(c % ntx, c / ntx, true), out = cost(c % ntx, c / ntx, false);
+        double acc = 0.0;
+        int from = 0, k = 1;
+        for (int i = 0; i < Nz; i++) {
+            acc += inz[i] ? in : out;
+            if (i + 1 < Nz && !(k < best[c] && acc >= total[c] * k / best[c])) continue;
+            if ((int)rank.size() < k) rank.resize(k);
+            rank[k - 1].push_back(make_int4(c % ntx, c / ntx, from, i + 1));
+            from = i + 1;
+            k++;
+        }
+    }
+    for (const auto& r : rank) work.insert(work.end(), r.begin(), r.end());
+}
+
+template cudaError_t launch_step_march<float>(const MarchArgs<float>&, const SourceList<float>&, const int4*, int,
+                                              const long long*, int, cudaStream_t);
+template cudaError_t launch_step_march<double>(const MarchArgs<double>&, const SourceList<double>&, const int4*, int,
+                                               const long long*, int, cudaStream_t);
+template cudaError_t march_maps<float>(MarchArgs<float>&);
+template cudaError_t march_maps<double>(MarchArgs<double>&);
+template void march_work<float>(const GridView<float>&, int, int, std::vector<int4>&);
+template void march_work<double>(const GridView<double>&, int, int, std::vector<int4>&);
 
 }  // namespace fdtdb
