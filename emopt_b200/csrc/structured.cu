@@ -29,11 +29,18 @@
 // what remains after the last edge is the claimed piece.  Pieces smaller than
 // 1e-14 of the cell area are dropped.  Overflow of either limit is reported.
 //
-// One thread per output element; all arithmetic in float64.
+// A layer's value at a cell does not depend on z, so one thread evaluates a
+// column of up to kPlanes cells and works each layer out once per column, not
+// once per cell: the geometry (four corner tests against every primitive of the
+// layer, and the clipping of the cells on an outline) bounds the cell-by-cell
+// form, the 16 bytes written per cell bound this one away from the outlines.
+// All arithmetic in float64.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <vector>
 
 #include "../../include/emopt_fdtd.h"
 #include "common.cuh"
@@ -156,6 +163,8 @@ __device__ void layer_value(const Tables& t, int l, double xd, double yd, double
     for (int q = t.start[l]; q < t.start[l + 1]; q++) {
         const int pr = t.prims[q];
         const double* v = t.pval + 6 * pr;
+        // no corner of a cell beside the outline's bounding box is inside it
+        if (t.pinfo[4 * pr + 1] >= 0 && !(xmax > v[2] && xmin < v[3] && ymax > v[4] && ymin < v[5])) continue;
         const bool c1 = prim_contains(t, pr, xmin, ymin), c2 = prim_contains(t, pr, xmax, ymin);
         const bool c3 = prim_contains(t, pr, xmax, ymax), c4 = prim_contains(t, pr, xmin, ymax);
         if (c1 && c2 && c3 && c4 && area / max_area == 1.0) {
@@ -204,9 +213,23 @@ __device__ void layer_value(const Tables& t, int l, double xd, double yd, double
     if (area / max_area > 0.0) vr += area / max_area * 1.0;
 }
 
-// Value at fractional indices (x, y, z) (src/Grid.cpp:737-826).
-__device__ void material_value(const Tables& t, double x, double y, double z, double dx,
-                               double dy, double dz, double& vr, double& vi, int* err) {
+// The layer value of one column, kept while the column stays in the layer.
+struct LayerCache {
+    int l = -1;
+    double vr, vi;
+    __device__ __forceinline__ void get(const Tables& t, int layer, double xd, double yd, double dx, double dy,
+                                        int* err) {
+        if (layer == l) return;
+        layer_value(t, layer, xd, yd, dx, dy, vr, vi, err);
+        l = layer;
+    }
+};
+
+// Value at fractional indices (x, y, z) (src/Grid.cpp:737-826); (xd, yd) =
+// (x dx, y dy).  Layers below `from` end at or below this cell; `from` moves up
+// with the cells of a column.
+__device__ __forceinline__ void material_value(const Tables& t, double xd, double yd, double z, double dx, double dy,
+                                               double dz, int& from, LayerCache& c, double& vr, double& vi, int* err) {
     vr = 0.0;
     vi = 0.0;
     if (t.nz < 2) {
@@ -214,7 +237,6 @@ __device__ void material_value(const Tables& t, double x, double y, double z, do
         return;
     }
     double zmin = (z - 0.5) * dz, zmax = (z + 0.5) * dz;
-    const double xd = x * dx, yd = y * dy;
     if (zmax <= t.zs[0]) {
         vr = 1.0;
         return;
@@ -223,39 +245,53 @@ __device__ void material_value(const Tables& t, double x, double y, double z, do
         vr = (t.zs[0] - zmin) / dz * 1.0;
         zmin = t.zs[0];
     }
-    for (int l = 0; l + 1 < t.nz; l++) {
+    while (from + 1 < t.nz && t.zs[from + 1] <= zmin) from++;
+    for (int l = from; l + 1 < t.nz; l++) {
         const double za = t.zs[l], zb = t.zs[l + 1];
         if (zmin >= za && zmax <= zb) {
-            double lr, li;
-            layer_value(t, l, xd, yd, dx, dy, lr, li, err);
-            vr += (zmax - zmin) / dz * lr;
-            vi += (zmax - zmin) / dz * li;
+            c.get(t, l, xd, yd, dx, dy, err);
+            const double w = (zmax - zmin) / dz;
+            vr += w * c.vr;
+            vi += w * c.vi;
             return;
         } else if (zmin >= za && zmin < zb && zmax > zb) {
-            double lr, li;
-            layer_value(t, l, xd, yd, dx, dy, lr, li, err);
-            vr += (zb - zmin) / dz * lr;
-            vi += (zb - zmin) / dz * li;
+            c.get(t, l, xd, yd, dx, dy, err);
+            const double w = (zb - zmin) / dz;
+            vr += w * c.vr;
+            vi += w * c.vi;
             zmin = zb;
         }
     }
     vr += (zmax - zmin) / dz * 1.0;
 }
 
+// Cells of a column per thread: short enough that a small grid fills the chip,
+// long enough that a layer is evaluated for many cells at a time.
+constexpr int kPlanes = 16;
+
 __global__ void __launch_bounds__(128) k_structured(Tables t, double dx, double dy, double dz, int k1,
-                                                    int Nx, int j1, int Ny, int i1, long long n,
+                                                    int Nx, int j1, int i1, int Nz, long long cols,
                                                     double sx, double sy, double sz, c128* out,
-                                                    int* err) {
+                                                    bool aligned, int* err) {
     const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= n) return;
-    const long long row = q / Nx;
-    const int k = k1 + (int)(q - row * Nx);
-    const int j = j1 + (int)(row % Ny);
-    const int i = i1 + (int)(row / Ny);
-    double vr, vi;
-    material_value(t, k + sx, j + sy, i + sz, dx, dy, dz, vr, vi, err);
-    out[q].real = vr;
-    out[q].imag = vi;
+    if (q >= cols) return;
+    const int j = j1 + (int)(q / Nx);
+    const int k = k1 + (int)(q % Nx);
+    const double xd = (k + sx) * dx, yd = (j + sy) * dy;
+    const int a = (int)blockIdx.y * kPlanes, b = min(a + kPlanes, Nz);
+    LayerCache c;
+    int from = 0;
+    for (int i = a; i < b; i++) {
+        double vr, vi;
+        material_value(t, xd, yd, (i1 + i) + sz, dx, dy, dz, from, c, vr, vi, err);
+        c128* const p = out + (long long)i * cols + q;
+        if (aligned) {
+            *reinterpret_cast<double2*>(p) = make_double2(vr, vi);
+        } else {
+            p->real = vr;
+            p->imag = vi;
+        }
+    }
 }
 
 }  // namespace
@@ -337,17 +373,21 @@ extern "C" int FDTD_structured_values(int device, void* stream, const double* zs
     unsigned char* pq = pv + up(bv);
     unsigned char* px = pq + up(bq);
     int* perr = reinterpret_cast<int*>(px + up(bx));
-    auto put = [&](void* dst, const void* src, size_t bytes) {
-        if (e == cudaSuccess && bytes > 0 && src) e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, st);
+    // all tables and the cleared error word in one copy
+    std::vector<unsigned char> host(total, 0);
+    auto put = [&](unsigned char* dst, const void* src, size_t bytes) {
+        if (bytes > 0 && src) std::memcpy(host.data() + (dst - d), src, bytes);
     };
-    put(pz, zs, sizeof(double) * (size_t)nzs);
-    if (nlayers > 0) put(ps, layer_start, bs);
-    put(pp, layer_prims, sizeof(int) * (size_t)nref);
-    put(pi, prim_info, sizeof(int) * 4 * (size_t)nprims);
-    put(pv, prim_vals, sizeof(double) * 6 * (size_t)nprims);
-    put(pq, parts, sizeof(int) * 2 * (size_t)nparts);
-    put(px, verts, sizeof(double) * 2 * (size_t)nverts);
-    if (e == cudaSuccess) e = cudaMemsetAsync(perr, 0, sizeof(int), st);
+    if (e == cudaSuccess) {
+        put(pz, zs, sizeof(double) * (size_t)nzs);
+        if (nlayers > 0) put(ps, layer_start, bs);
+        put(pp, layer_prims, sizeof(int) * (size_t)nref);
+        put(pi, prim_info, sizeof(int) * 4 * (size_t)nprims);
+        put(pv, prim_vals, sizeof(double) * 6 * (size_t)nprims);
+        put(pq, parts, sizeof(int) * 2 * (size_t)nparts);
+        put(px, verts, sizeof(double) * 2 * (size_t)nverts);
+        e = cudaMemcpyAsync(d, host.data(), total, cudaMemcpyDefault, st);
+    }
     int herr = 0;
     if (e == cudaSuccess) {
         fdtdb::Tables t;
@@ -360,10 +400,16 @@ extern "C" int FDTD_structured_values(int device, void* stream, const double* zs
         t.parts = reinterpret_cast<const int*>(pq);
         t.verts = reinterpret_cast<const double*>(px);
         fdtdb::c128* o = out_dev ? reinterpret_cast<fdtdb::c128*>(out) : dout;
-        const unsigned grid = (unsigned)((n + 127) / 128);
-        fdtdb::k_structured<<<grid, 128, 0, st>>>(t, dx, dy, dz, k1, (int)Nx, j1, (int)Ny, i1, n, sx,
-                                                  sy, sz, o, perr);
-        e = cudaGetLastError();
+        const long long cols = Nx * Ny;
+        // the y extent of a launch is bounded, so very deep ranges take several
+        const long long step = 65535LL * fdtdb::kPlanes;
+        for (long long i = 0; i < Nz && e == cudaSuccess; i += step) {
+            const int nz = (int)std::min(step, Nz - i);
+            const dim3 grid((unsigned)((cols + 127) / 128), (unsigned)((nz + fdtdb::kPlanes - 1) / fdtdb::kPlanes));
+            fdtdb::k_structured<<<grid, 128, 0, st>>>(t, dx, dy, dz, k1, (int)Nx, j1, i1 + (int)i, nz, cols, sx, sy, sz,
+                                                      o + i * cols, (reinterpret_cast<uintptr_t>(o) & 15) == 0, perr);
+            e = cudaGetLastError();
+        }
         if (e == cudaSuccess && !out_dev)
             e = cudaMemcpyAsync(out, dout, sizeof(fdtdb::c128) * (size_t)n, cudaMemcpyDefault, st);
         if (e == cudaSuccess) e = cudaMemcpyAsync(&herr, perr, sizeof(int), cudaMemcpyDefault, st);

@@ -164,17 +164,24 @@ class Polygon(MaterialPrimitive):
         self._xs[index] = x
         self._ys[index] = y
 
-    def outline(self):
-        """Vertices counter-clockwise, without a repeated closing vertex."""
-        x, y = self._xs, self._ys
+    def _vertices(self):
+        """The outline as a list of [x, y], counter-clockwise, without a
+        repeated closing vertex."""
+        x, y = self._xs.tolist(), self._ys.tolist()
         if len(x) > 1 and x[0] == x[-1] and y[0] == y[-1]:
-            x, y = x[:-1], y[:-1]
+            del x[-1], y[-1]
         if len(x) < 3:
             raise ValueError("a Polygon needs at least 3 vertices")
-        area2 = np.sum(x * np.roll(y, -1) - np.roll(x, -1) * y)
-        if area2 < 0:
-            x, y = x[::-1], y[::-1]
-        return np.stack([x, y], axis=1)
+        terms = [a * d - c * b for a, b, c, d in zip(x, y, x[1:] + x[:1], y[1:] + y[:1])]
+        area2 = sum(terms)
+        if not abs(area2) > 1e-9 * sum(map(abs, terms)):
+            area2 = np.sum(terms)       # nearly flat: the sign of numpy's sum decides
+        v = [list(p) for p in zip(x, y)]
+        return v[::-1] if area2 < 0 else v
+
+    def outline(self):
+        """Vertices counter-clockwise, without a repeated closing vertex."""
+        return np.array(self._vertices())
 
     def contains_point(self, x, y):
         v = self.outline()
@@ -190,13 +197,15 @@ class Polygon(MaterialPrimitive):
 
 
 def _convex_parts(v):
-    """Convex pieces of the counter-clockwise outline v: itself when convex,
+    """Convex pieces of the counter-clockwise outline v (a list of [x, y]): itself when convex,
     else the triangles of an ear-clipping triangulation."""
     n = len(v)
-    cross = [(v[(q + 1) % n][0] - v[q][0]) * (v[(q + 2) % n][1] - v[(q + 1) % n][1]) -
-             (v[(q + 1) % n][1] - v[q][1]) * (v[(q + 2) % n][0] - v[(q + 1) % n][0]) for q in range(n)]
-    if all(c >= 0 for c in cross):
+    w = v if isinstance(v, list) else np.asarray(v).tolist()      # plain floats: cheaper to index
+    w = w + w[:2]
+    if all((b[0] - a[0]) * (c[1] - b[1]) - (b[1] - a[1]) * (c[0] - b[0]) >= 0
+           for a, b, c in zip(w, w[1:], w[2:])):
         return [v]
+    v = np.asarray(v)
     idx = list(range(n))
     tris = []
 
@@ -371,21 +380,21 @@ class StructuredMaterial3D(Material3D):
                 continue
             if isinstance(p, Rectangle):
                 x0, x1, y0, y1 = p.bounds()
-                outline = np.array([[x0, y0], [x1, y0], [x1, y1], [x0, y1]])
+                outline = [[x0, y0], [x1, y0], [x1, y1], [x0, y1]]
                 pieces = [outline]
             else:
-                outline = p.outline()
+                outline = p._vertices()
                 pieces = _convex_parts(outline)
             ov = len(verts)
-            verts.extend(outline.tolist())
+            verts.extend(outline)
             pp = len(parts)
             for piece in pieces:
                 parts.append((len(verts), len(piece)))
-                verts.extend(np.asarray(piece).tolist())
+                verts.extend(piece if piece is outline else piece.tolist())
             info.append((ov, len(outline), pp, len(pieces)))
             m = complex(p.material_value)
-            vals.append((m.real, m.imag, outline[:, 0].min(), outline[:, 0].max(),
-                         outline[:, 1].min(), outline[:, 1].max()))
+            xs, ys = [q[0] for q in outline], [q[1] for q in outline]
+            vals.append((m.real, m.imag, min(xs), max(xs), min(ys), max(ys)))
         i32 = lambda a, w: np.asarray(a if len(a) else [[0] * w], dtype=np.int32).reshape(-1)
         return (np.asarray(self._zs, dtype=np.float64), np.asarray(start, dtype=np.int32),
                 np.asarray(flat if flat else [0], dtype=np.int32), i32(info, 4),
