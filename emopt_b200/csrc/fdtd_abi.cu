@@ -66,6 +66,7 @@ struct HostSource {
 template <typename T>
 struct Resident {
     int Nx = 0, Ny = 0, Nz = 0, px = 0;
+    DevBuf arena;            // the one allocation that alloc_resident cuts into the arrays
     DevBuf F[2][6];          // fields Ex Ey Ez Hx Hy Hz; set 1: the fused step's second set
     DevBuf bE[3], aE[3], bH[3];
     bool mu_uniform[3] = {true, true, true};
@@ -100,6 +101,7 @@ struct Resident {
         steptab.release(); stepbase.release(); flag.release(); err.release();
         pwin.release(); pA.release(); pphi.release(); ptimes.release(); pout.release(); pmap.release();
         psamp.release();
+        arena.release();
         coeffs_valid = false;
         Nx = Ny = Nz = px = 0;
         halo = 0;
@@ -821,25 +823,45 @@ bool march_possible(const FDTDHandle* h) {
 template <typename T>
 int alloc_resident(FDTDHandle* h, Resident<T>& r, bool march, int halo = 0) {
     int px = (h->Nx + 31) / 32 * 32;
-    bool same = r.Nx == h->Nx && r.Ny == h->Ny && r.Nz == h->Nz && r.px == px && r.halo == halo;
-    if (!same) r.release_all();
-    r.Nx = h->Nx; r.Ny = h->Ny; r.Nz = h->Nz; r.px = px; r.halo = halo;
     size_t cells = (size_t)h->Nz * h->Ny * px;
     size_t fcells = (size_t)(h->Nz + 2 * halo) * h->Ny * px;
     long long slab[3] = {(long long)h->Nz * h->Ny * (march ? x_slab<T>(h).pitch : h->w[0] + h->w[1]),
                          (long long)h->Nz * (h->w[2] + h->w[3]) * px,
                          (long long)(h->w[4] + h->w[5]) * h->Ny * px};
+    // One allocation holds all of them: allocating and freeing the ~35 arrays of
+    // a served request one by one cost about 10 ms each way.
+    struct Want { DevBuf* b; size_t bytes; };
+    std::vector<Want> want;
     for (int s = 0; s < (march ? 2 : 1); s++) {
-        for (int c = 0; c < 6; c++) CK(r.F[s][c].ensure(sizeof(T) * fcells));
+        for (int c = 0; c < 6; c++) want.push_back({&r.F[s][c], sizeof(T) * fcells});
         for (int a = 0; a < 3; a++)
-            for (int q = 0; q < (s ? 2 : 4); q++) CK(r.psi[s][a][q].ensure(sizeof(T) * (slab[a] ? slab[a] : 1)));
+            for (int q = 0; q < (s ? 2 : 4); q++) want.push_back({&r.psi[s][a][q], sizeof(T) * (size_t)(slab[a] ? slab[a] : 1)});
     }
-    for (int c = 0; c < 3; c++) CK(r.bE[c].ensure(sizeof(T) * cells));
+    for (int c = 0; c < 3; c++) want.push_back({&r.bE[c], sizeof(T) * cells});
     for (int s = 0; s < 2; s++)
-        for (int c = 0; c < 6; c++) CK(r.snap[s][c].ensure(sizeof(T) * cells));
-    CK(r.stepbase.ensure(sizeof(long long)));
-    CK(r.flag.ensure(sizeof(int) * 4));
-    CK(r.err.ensure(sizeof(int) * 4));
+        for (int c = 0; c < 6; c++) want.push_back({&r.snap[s][c], sizeof(T) * cells});
+    want.push_back({&r.stage, sizeof(c128) * (size_t)h->Nx * h->Ny * h->Nz});
+    want.push_back({&r.stepbase, sizeof(long long)});
+    want.push_back({&r.flag, sizeof(int) * 4});
+    want.push_back({&r.err, sizeof(int) * 4});
+    auto up = [](size_t n) { return (n + 511) / 512 * 512; };
+    size_t total = 0;
+    bool same = r.Nx == h->Nx && r.Ny == h->Ny && r.Nz == h->Nz && r.px == px && r.halo == halo;
+    for (const Want& w : want) {
+        total += up(w.bytes);
+        same = same && w.b->p && w.b->bytes >= w.bytes;
+    }
+    if (same) return FDTD_OK;
+    r.release_all();
+    CK(r.arena.ensure(total));
+    r.Nx = h->Nx; r.Ny = h->Ny; r.Nz = h->Nz; r.px = px; r.halo = halo;
+    size_t at = 0;
+    for (const Want& w : want) {
+        w.b->p = (unsigned char*)r.arena.p + at;
+        w.b->bytes = w.bytes;
+        w.b->owned = false;
+        at += up(w.bytes);
+    }
     return FDTD_OK;
 }
 
