@@ -1146,9 +1146,8 @@ int solve_impl(FDTDHandle* h, const FDTDSolveOptions* o, FDTDSolveResult* res) {
     // kernel ids: 0 auto, 1 scalar H/E pair, 3 fused step, 5 vector H/E pair, 6
     // vector pair split into interior and rim launches.  Auto takes the fused
     // step wherever it is possible but for rows of at most 16 vectors, which
-    // leave half of its lanes idle (64 x 64 x 64 in float32: 16.6 us per step
-    // against 14.6 for the vector pair; 72 x 72 x 72: 18.2 against 22.7; in
-    // float64, 64 x 64 x 64: 16.8 against 18.9).  Without it: the split pair in
+    // leave half of its lanes idle (56 x 48 x 44 in float32: 12.6 us per step
+    // either way; 72 x 72 x 72: 18.2 against 22.7).  Without it: the split pair in
     // float32 when at least 60% of the warp tasks lie in no CPML slab (the
     // 1201 x 601 x 301 grating slab, 69%: 3293 instead of 3605 us per step;
     // the 321 x 161 x 101 MMI block, 23%: 143 instead of 122), else the

@@ -26,10 +26,15 @@
 // 113 KB of shared memory and 128 registers leave, and any register spilled
 // inside the plane loop costs more than it saves (the L1 is all shared memory:
 // 16 bytes spilled took 193 us instead of 126).  us per step, before (vector
-// pair, in the large slab the interior/rim pair) and now, 15- or 20-cell slabs:
-//   float32  96x80x72 22.8 -> 18.7, 128x128x96 39.2 -> 31.0, 321x161x101
-//            122.8 -> 105.6, 801x401x201 1043 -> 920
-//   float64  101x76x65 27.0 -> 24.9, 321x161x101 207.5 -> 185
+// pair, in the large slab the interior/rim pair) and now, 10- to 20-cell slabs:
+//   float32  80x80x80 24.9 -> 17.2, 161x81x51 22.9 -> 20.0, 321x161x101 122.8 ->
+//            105.0, 801x401x201 1043 -> 905
+//   float64  101x76x65 27.0 -> 23.9, 161x81x51 28.9 -> 27.7, 321x161x101 207.5 ->
+//            184.7
+// Steps are launched with programmatic serialization: a step's CTAs start up in
+// the slots the last CTAs of the step before leave and wait there for its end
+// (16.6 -> 14.4 us on 64x64x64, 21.2 -> 20.0 on 161x81x51 in float32, 920 -> 905
+// on the slab).
 #include <algorithm>
 #include <cmath>
 #include <queue>
@@ -250,7 +255,18 @@ k_step_march(const __grid_constant__ MarchArgs<T> A, const __grid_constant__ Sou
     const PmlAxis<T>& PY = g.pml[1];
     const PmlAxis<T>& PZ = g.pml[2];
     const int lane = threadIdx.x & 31, w = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
-    const int4 job = __ldg(work + blockIdx.x);      // x tile, row tile, planes job.z .. job.w - 1
+    // The next step may take the slots this one leaves (its copies wait below for
+    // the whole of this grid), so its start-up overlaps this step's last CTAs.
+    asm volatile("griddepcontrol.launch_dependents;");
+    const unsigned bars = smem_u32(smem) + L::bars;
+    const bool leader = threadIdx.x == 0;
+    if (leader) {
+        for (int q = 0; q < 4; q++) mbar_init(bars + 8 * q);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    const int4 job = work[blockIdx.x];              // x tile, row tile, planes job.z .. job.w - 1
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("fence.proxy.async.global;" ::: "memory");   // the box copies read what the last step stored
     const int x0 = job.x * (30 * VW), c0 = x0 + lane * VW;
     const int j0 = job.y * R, j = j0 - 1 + w;
     const int i0 = job.z, i1 = job.w, is = i0 > 0 ? i0 - 1 : 0;
@@ -260,7 +276,7 @@ k_step_march(const __grid_constant__ MarchArgs<T> A, const __grid_constant__ Sou
     // byte offsets: a plane, this vector in a plane
     const unsigned pb = (unsigned)g.Ny * g.px * SZ;
     const unsigned rb = ok ? (unsigned)(j * g.px + c0) * SZ : 0u;
-    const unsigned sbase = smem_u32(smem), bars = sbase + L::bars;
+    const unsigned sbase = smem_u32(smem);
     const int ly = row ? slab_local(PY, j, false) : -1;
     // x slab: slot of this vector in the whole-vector psi rows, or -1
     int sx = -1;
@@ -306,7 +322,6 @@ k_step_march(const __grid_constant__ MarchArgs<T> A, const __grid_constant__ Sou
     // Copies of one thread: E of plane p (Ez unless only read from below) into
     // a ring slot; Ey of plane p and H of plane q into their stages; the
     // coefficients of plane q.
-    const bool leader = threadIdx.x == 0;
     auto stage_at = [&](int i) { return sbase + L::stage0 + (((i - is) & 1) ? L::stage : 0u); };
     auto fetch_e = [&](int p, unsigned slot, bool full, unsigned bar) {
         tma_box(slot, &A.tm_in[0], x0, j0 - 1, p, bar);
@@ -340,8 +355,6 @@ k_step_march(const __grid_constant__ MarchArgs<T> A, const __grid_constant__ Sou
     unsigned r0 = sbase, r1 = sbase + L::ring, r2 = sbase + 2 * L::ring;
     unsigned sa = sbase + L::stage0, sb = sa + L::stage, ba = bars, bb = bars + 8;
     if (leader) {
-        for (int q = 0; q < 4; q++) mbar_init(bars + 8 * q);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         // E(is), E(is+1), H(is) for the first plane; E(is+2), H(is+1) for the next
         mbar_expect(ba, a_bytes + 2 * (NW + 1) * kRow - (is + 1 < i1 ? 0 : (NW + 1) * kRow));
         fetch_e(is, r0, true, ba);
@@ -410,6 +423,8 @@ k_step_march(const __grid_constant__ MarchArgs<T> A, const __grid_constant__ Sou
         // ---- E of the plane, the row above and the plane above; H
         wait(ba, phase);
         if (i + 1 < i1) {
+            if (MUARR && ok)
+                for (int c = 0; c < 3; c++) l1_prefetch(at(g.bHarr[c], o + pb));
             if (iny) { l1_prefetch(at(A.ph_in[1][0], oY + strideY)); l1_prefetch(at(A.ph_in[1][1], oY + strideY)); }
             if (inz) { l1_prefetch(at(A.ph_in[2][0], oZ + pb)); l1_prefetch(at(A.ph_in[2][1], oZ + pb)); }
         }
@@ -472,6 +487,8 @@ k_step_march(const __grid_constant__ MarchArgs<T> A, const __grid_constant__ Sou
         // ---- CPML state of the E update
         if (iny) { py0 = gload(at(A.pe[1][0], oY), eo); py1 = gload(at(A.pe[1][1], oY), eo); }
         if (inz) { pz0 = gload(at(A.pe[2][0], oZ), eo); pz1 = gload(at(A.pe[2][1], oZ), eo); }
+        V a0, a1, a2;                                  // E-update factors of lossy media
+        if (LOSSY) { a0 = gload(at(g.aE[0], o), eo); a1 = gload(at(g.aE[1], o), eo); a2 = gload(at(g.aE[2], o), eo); }
         __syncthreads();
         // E(i), Ey(i+1), H(i) and the coefficients of plane i - 1 have been read:
         // the next copies, spread over the warps (one issue takes ~200 cycles)
@@ -520,9 +537,9 @@ k_step_march(const __grid_constant__ MarchArgs<T> A, const __grid_constant__ Sou
                 V t[3] = {pk::mul(oz, fydz), pk::mul(ox, fzdx), pk::mul(oy, fxdy)};
                 curls<T>(modeE, plE, oA, fA, t, mone);
                 if (LOSSY) {
-                    ex = pk::fma(gload(at(g.aE[0], o), ownu), ex, pk::mul(t[0], bx));
-                    ey = pk::fma(gload(at(g.aE[1], o), ownu), ey, pk::mul(t[1], by));
-                    ez = pk::fma(gload(at(g.aE[2], o), ownu), ez, pk::mul(t[2], bz));
+                    ex = pk::fma(a0, ex, pk::mul(t[0], bx));
+                    ey = pk::fma(a1, ey, pk::mul(t[1], by));
+                    ez = pk::fma(a2, ez, pk::mul(t[2], bz));
                 } else {
                     ex = pk::fma(t[0], bx, ex); ey = pk::fma(t[1], by, ey); ez = pk::fma(t[2], bz, ez);
                 }
@@ -584,8 +601,17 @@ cudaError_t launch_one(const MarchArgs<T>& a, const SourceList<T>& src, const in
     auto k = k_step_march<T, kNW, kMinB, LOSSY, MUARR>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return e;
-    k<<<nwork, 32 * kNW, bytes, st>>>(a, src, work, step_base, off);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(nwork);
+    cfg.blockDim = dim3(32 * kNW);
+    cfg.dynamicSmemBytes = bytes;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k, a, src, work, step_base, off);
 }
 
 template <typename T>
