@@ -72,7 +72,7 @@ def build(verbose: bool = False, force: bool = False, checked: bool = True) -> s
     """Build FDTD.so (and, unless ``checked`` is False, FDTD_checked.so)."""
     os.makedirs(BUILD, exist_ok=True)
     headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))]
-    headers.append(os.path.join(os.path.dirname(HERE), "include", "emopt_fdtd.h"))
+    headers += [os.path.join(os.path.dirname(HERE), "include", f) for f in ("emopt_fdtd.h", "emopt_modes.h")]
     objs = []
     for src in SOURCES:
         o = os.path.join(BUILD, src.replace(".cu", ".o"))

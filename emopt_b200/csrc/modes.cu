@@ -22,10 +22,12 @@
 // line l, component c (Ex Ey Ez Hx Hy Hz) and position p along the line.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 
 #include "../../include/emopt_fdtd.h"
+#include "../../include/emopt_modes.h"
 
 namespace modes {
 
@@ -253,6 +255,257 @@ __global__ void __launch_bounds__(256) k_lines_gemv(int nb, const double* W, con
     }
 }
 
+// ---- In-place inverses of the line blocks W[line] (nb x nb, row major) by
+// blocked Gauss-Jordan elimination with partial pivoting (Householder 1964;
+// Quintana-Orti et al. 2001), panels of B columns.  With K the panel's columns,
+// A' the matrix after the panel's row exchanges and G the panel after the
+// elimination of its B columns over all rows (G_K = A'_KK^-1, G_i = -A'_iK G_K),
+// every other column j becomes A_ij = (i in K ? 0 : A'_ij) + G_i A'_Kj.  Three
+// kernels per panel: the panel in shared memory, one CTA per matrix (a serial
+// chain of B pivot steps, the bound where a level holds few lines); the row
+// exchanges of the other columns, which also take out A'_K; the update, a rank-B
+// product per 64 x 64 tile (the bound of the first levels: it reads and writes
+// the matrix once per panel).  The column exchanges follow at the end.
+
+// A panel's row exchanges: row dst[q] receives the old row src[q], the panel's
+// rows first.
+template <int B>
+struct Moves {
+    int n;
+    int dst[2 * B], src[2 * B];
+};
+
+// 1 / z, scaled against overflow (Smith 1962).
+__device__ __forceinline__ C2 recip(C2 z) {
+    if (fabs(z.x) >= fabs(z.y)) {
+        const double r = z.y / z.x, d = z.x + z.y * r;
+        return {1.0 / d, -r / d};
+    }
+    const double r = z.x / z.y, d = z.x * r + z.y;
+    return {r / d, -1.0 / d};
+}
+
+template <int B>
+__global__ void __launch_bounds__(1024) k_inv_panel(int n, double* W, const int* lines, int k0, int* piv,
+                                                    Moves<B>* moves, int* info) {
+    extern __shared__ double2 P[];                    // n rows of B + 1: rows 16 (B + 1) bytes apart, no bank conflicts
+    __shared__ double best[32];
+    __shared__ int where[32];
+    const int z = blockIdx.x, b = min(B, n - k0);
+    double2* A = reinterpret_cast<double2*>(W) + (long long)lines[z] * n * n;
+    int* pv = piv + (long long)z * n;
+    for (int t = threadIdx.x; t < n * b; t += blockDim.x) {
+        const int r = t / b, c = t - r * b;
+        P[r * (B + 1) + c] = A[(long long)r * n + k0 + c];
+    }
+    __syncthreads();
+    for (int c = 0; c < b; c++) {
+        const int k = k0 + c;
+        double m = -1.0;
+        int at = k;
+        for (int r = threadIdx.x; r < n; r += blockDim.x) {
+            if (r < k) continue;
+            const double2 v = P[r * (B + 1) + c];
+            const double a = fabs(v.x) + fabs(v.y);
+            if (a > m) { m = a; at = r; }
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            const double m2 = __shfl_xor_sync(0xffffffffu, m, o);
+            const int a2 = __shfl_xor_sync(0xffffffffu, at, o);
+            if (m2 > m || (m2 == m && a2 < at)) { m = m2; at = a2; }
+        }
+        if ((threadIdx.x & 31) == 0) { best[threadIdx.x >> 5] = m; where[threadIdx.x >> 5] = at; }
+        __syncthreads();
+        m = best[0];
+        at = where[0];
+        for (int q = 1; q < (int)(blockDim.x >> 5); q++)
+            if (best[q] > m || (best[q] == m && where[q] < at)) { m = best[q]; at = where[q]; }
+        if (threadIdx.x == 0) {
+            pv[k] = at;
+            if (!(m > 0.0) || isinf(m)) info[z] = 1;
+        }
+        // exchange rows k and at, then the pivot row times 1 / pivot (its own
+        // column becomes 1 / pivot)
+        if ((int)threadIdx.x < 32) {
+            const int q = threadIdx.x;
+            double2 x = make_double2(0, 0), y = x;
+            if (q < b) { x = P[k * (B + 1) + q]; y = P[at * (B + 1) + q]; }
+            C2 d = {__shfl_sync(0xffffffffu, y.x, c), __shfl_sync(0xffffffffu, y.y, c)};
+            d = recip(d);
+            if (q < b) {
+                if (at != k) P[at * (B + 1) + q] = x;
+                const C2 v = q == c ? d : d * C2{y.x, y.y};
+                P[k * (B + 1) + q] = make_double2(v.x, v.y);
+            }
+        }
+        __syncthreads();
+        for (int r = threadIdx.x; r < n; r += blockDim.x) {
+            if (r == k) continue;
+            double2* row = P + r * (B + 1);
+            const double2 f = row[c];
+#pragma unroll
+            for (int q = 0; q < B; q++) {
+                if (q >= b) break;
+                const double2 u = P[k * (B + 1) + q];
+                double2 a = q == c ? make_double2(0.0, 0.0) : row[q];
+                a.x = fma(-f.x, u.x, fma(f.y, u.y, a.x));
+                a.y = fma(-f.x, u.y, fma(-f.y, u.x, a.y));
+                row[q] = a;
+            }
+        }
+        __syncthreads();
+    }
+    for (int t = threadIdx.x; t < n * b; t += blockDim.x) {
+        const int r = t / b, c = t - r * b;
+        A[(long long)r * n + k0 + c] = P[r * (B + 1) + c];
+    }
+    if (threadIdx.x == 0) {
+        // where each moved row's content comes from
+        Moves<B>& M = moves[z];
+        int cnt = b;
+        for (int c = 0; c < b; c++) M.dst[c] = M.src[c] = k0 + c;
+        for (int c = 0; c < b; c++) {
+            const int p = pv[k0 + c];
+            int q = 0;
+            while (q < cnt && M.dst[q] != p) q++;
+            if (q == cnt) { M.dst[cnt] = M.src[cnt] = p; cnt++; }
+            const int t = M.src[c];
+            M.src[c] = M.src[q];
+            M.src[q] = t;
+        }
+        M.n = cnt;
+    }
+}
+
+// Row exchanges of the columns outside the panel; the panel's rows go to R
+// (B x n per matrix), the update rewrites them.
+template <int B>
+__global__ void __launch_bounds__(128) k_inv_swap(int n, double* W, const int* lines, int k0, const Moves<B>* moves,
+                                                  double2* R) {
+    const int z = blockIdx.y, j = blockIdx.x * 128 + threadIdx.x, b = min(B, n - k0);
+    if (j >= n || (j >= k0 && j < k0 + b)) return;
+    double2* A = reinterpret_cast<double2*>(W) + (long long)lines[z] * n * n + j;
+    const Moves<B>& M = moves[z];
+    double2 v[2 * B];
+#pragma unroll
+    for (int q = 0; q < 2 * B; q++)
+        if (q < M.n) v[q] = A[(long long)M.src[q] * n];
+    double2* Rz = R + ((long long)z * B) * n + j;
+#pragma unroll
+    for (int q = 0; q < 2 * B; q++) {
+        if (q >= M.n) break;
+        if (q < b) Rz[(long long)q * n] = v[q];
+        else A[(long long)M.dst[q] * n] = v[q];
+    }
+}
+
+// A_ij = (i in K ? 0 : A_ij) + G_i R_j for the columns j outside the panel K.
+// 16 x 16 threads, 4 x 4 values each, 16 rows or columns apart (a quarter warp
+// reads 128 consecutive bytes).
+template <int B>
+__global__ void __launch_bounds__(256) k_inv_update(int n, double* W, const int* lines, int k0, const double2* R) {
+    __shared__ double2 G[B][64 + 1], U[B][64];
+    const int z = blockIdx.z, b = min(B, n - k0);
+    double2* A = reinterpret_cast<double2*>(W) + (long long)lines[z] * n * n;
+    const int i0 = blockIdx.y * 64, j0 = blockIdx.x * 64, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    for (int t = threadIdx.x; t < 64 * B; t += 256) {
+        const int r = t / B, c = t - r * B;
+        G[c][r] = i0 + r < n && c < b ? A[(long long)(i0 + r) * n + k0 + c] : make_double2(0, 0);
+        const int q = t / 64, j = t - q * 64;
+        U[q][j] = j0 + j < n && q < b ? R[((long long)z * B + q) * n + j0 + j] : make_double2(0, 0);
+    }
+    double2 a[4][4];
+#pragma unroll
+    for (int ii = 0; ii < 4; ii++)
+#pragma unroll
+        for (int jj = 0; jj < 4; jj++) {
+            const int i = i0 + ty + 16 * ii, j = j0 + tx + 16 * jj;
+            a[ii][jj] = i < n && j < n && (i < k0 || i >= k0 + b) ? A[(long long)i * n + j] : make_double2(0, 0);
+        }
+    __syncthreads();
+#pragma unroll 4
+    for (int q = 0; q < B; q++) {
+        double2 g[4], u[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) { g[e] = G[q][ty + 16 * e]; u[e] = U[q][tx + 16 * e]; }
+#pragma unroll
+        for (int ii = 0; ii < 4; ii++)
+#pragma unroll
+            for (int jj = 0; jj < 4; jj++) {
+                a[ii][jj].x = fma(g[ii].x, u[jj].x, fma(-g[ii].y, u[jj].y, a[ii][jj].x));
+                a[ii][jj].y = fma(g[ii].x, u[jj].y, fma(g[ii].y, u[jj].x, a[ii][jj].y));
+            }
+    }
+#pragma unroll
+    for (int ii = 0; ii < 4; ii++)
+#pragma unroll
+        for (int jj = 0; jj < 4; jj++) {
+            const int i = i0 + ty + 16 * ii, j = j0 + tx + 16 * jj;
+            if (i < n && j < n && (j < k0 || j >= k0 + b)) A[(long long)i * n + j] = a[ii][jj];
+        }
+}
+
+// perm[j]: the column of the eliminated matrix that ends at column j (the row
+// exchanges undone on the columns, last first).
+__global__ void k_inv_perm(int n, const int* piv, int* perm) {
+    extern __shared__ int col[];
+    const int* pv = piv + (long long)blockIdx.x * n;
+    for (int t = threadIdx.x; t < n; t += blockDim.x) col[t] = t;
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int k = n - 1; k >= 0; k--) {
+            const int p = pv[k], t = col[k];
+            col[k] = col[p];
+            col[p] = t;
+        }
+    __syncthreads();
+    for (int t = threadIdx.x; t < n; t += blockDim.x) perm[(long long)blockIdx.x * n + t] = col[t];
+}
+
+__global__ void __launch_bounds__(256) k_inv_columns(int n, double* W, const int* lines, const int* perm) {
+    extern __shared__ double2 row[];
+    double2* A = reinterpret_cast<double2*>(W) + ((long long)lines[blockIdx.y] * n + blockIdx.x) * n;
+    const int* pm = perm + (long long)blockIdx.y * n;
+    for (int j = threadIdx.x; j < n; j += blockDim.x) row[j] = A[j];
+    __syncthreads();
+    for (int j = threadIdx.x; j < n; j += blockDim.x) A[j] = row[pm[j]];
+}
+
+constexpr size_t kInvSmem = 225 * 1024;              // shared memory of the panel kernel
+template <int B>
+size_t panel_bytes(int n) { return sizeof(double2) * (size_t)n * (B + 1); }
+
+// Work memory of the inverses of nl matrices: R, the moves, pivots, permutation.
+size_t inv_work(int n, int nl) {
+    auto up = [](size_t x) { return (x + 255) / 256 * 256; };
+    return up(sizeof(double2) * 16 * (size_t)n * nl) + up(sizeof(Moves<16>) * (size_t)nl) + 2 * up(sizeof(int) * (size_t)n * nl);
+}
+
+template <int B>
+cudaError_t invert(int n, double* W, const int* lines, int nl, unsigned char* work, int* info, cudaStream_t st) {
+    auto up = [](size_t x) { return (x + 255) / 256 * 256; };
+    double2* R = reinterpret_cast<double2*>(work);
+    Moves<B>* mv = reinterpret_cast<Moves<B>*>(work + up(sizeof(double2) * 16 * (size_t)n * nl));
+    int* piv = reinterpret_cast<int*>(reinterpret_cast<unsigned char*>(mv) + up(sizeof(Moves<16>) * (size_t)nl));
+    int* perm = reinterpret_cast<int*>(reinterpret_cast<unsigned char*>(piv) + up(sizeof(int) * (size_t)n * nl));
+    cudaError_t e = cudaMemsetAsync(info, 0, sizeof(int) * nl, st);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_inv_panel<B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInvSmem);
+    const int threads = std::min(1024, (n + 31) / 32 * 32), tiles = (n + 63) / 64;
+    for (int k0 = 0; k0 < n && e == cudaSuccess; k0 += B) {
+        k_inv_panel<B><<<nl, threads, panel_bytes<B>(n), st>>>(n, W, lines, k0, piv, mv, info);
+        if (n > B) {
+            k_inv_swap<B><<<dim3((n + 127) / 128, nl), 128, 0, st>>>(n, W, lines, k0, mv, R);
+            k_inv_update<B><<<dim3(tiles, tiles, nl), 256, 0, st>>>(n, W, lines, k0, R);
+        }
+        e = cudaGetLastError();
+    }
+    if (e != cudaSuccess) return e;
+    k_inv_perm<<<nl, 256, sizeof(int) * n, st>>>(n, piv, perm);
+    k_inv_columns<<<dim3(n, nl), 256, sizeof(double2) * n, st>>>(n, W, lines, perm);
+    return cudaGetLastError();
+}
+
 // Couplings between lines, batched: for z < nlines,
 //   dst[lines[z]][rows[i]] += sign * sum_j C[z][i][j] src[nbrs[z]][cols[j]]
 // (C: nlines x R x Q, dense).  A warp per (z, i); lanes walk j.  Every
@@ -404,6 +657,26 @@ int FDTD_mode_lines_gemv(int nb, int device, void* stream, const double* W, cons
     dim3 grid(tiles, (unsigned)((nrows + 7) / 8), (unsigned)nlines);
     k_lines_gemv<<<grid, 256, 0, (cudaStream_t)stream>>>(nb, W, lines, rows, nrows, rhs, corr, out);
     MCK(cudaGetLastError(), "FDTD_mode_lines_gemv");
+    return FDTD_OK;
+}
+
+long long FDTD_mode_invert_work(int nb, int nlines) {
+    // columns per panel: as many as keep a panel in shared memory
+    if (nb < 1 || nlines < 1 || nlines > 65535 || panel_bytes<8>(nb) > kInvSmem) return 0;
+    return (long long)inv_work(nb, nlines);
+}
+
+int FDTD_mode_invert(int nb, int device, void* stream, double* W, const int* lines, int nlines, void* work,
+                     long long work_bytes, int* info) {
+    const long long need = FDTD_mode_invert_work(nb, nlines);
+    if (!W || !lines || !work || !info || need == 0 || work_bytes < need)
+        return fail(FDTD_ERR_ARG, "FDTD_mode_invert: bad arguments");
+    MCK(cudaSetDevice(device), "FDTD_mode_invert");
+    unsigned char* w = (unsigned char*)work;
+    cudaStream_t st = (cudaStream_t)stream;
+    MCK(panel_bytes<16>(nb) <= kInvSmem ? invert<16>(nb, W, lines, nlines, w, info, st)
+                                        : invert<8>(nb, W, lines, nlines, w, info, st),
+        "FDTD_mode_invert");
     return FDTD_OK;
 }
 

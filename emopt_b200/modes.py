@@ -38,6 +38,14 @@ _PERMUTE = {"x": {"Ex": "Ez", "Ey": "Ex", "Ez": "Ey", "Hx": "Hz", "Hy": "Hx", "H
 _BCS = ("0", "M", "E", "H", "P", "EM", "HM")
 
 
+# include/emopt_modes.h
+libFDTD.FDTD_mode_invert_work.argtypes = [ctypes.c_int, ctypes.c_int]
+libFDTD.FDTD_mode_invert_work.restype = ctypes.c_longlong
+libFDTD.FDTD_mode_invert.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
+                                     ctypes.c_int, ctypes.c_void_p, ctypes.c_longlong, ctypes.c_void_p]
+libFDTD.FDTD_mode_invert.restype = ctypes.c_int
+
+
 def _check(rc, what):
     if rc != _ct.FDTD_OK:
         raise _ct.FDTDError("%s: %s" % (what, libFDTD.FDTD_mode_last_error().decode()))
@@ -193,11 +201,23 @@ class ModeFullVector:
             Lc[1:, ar, ar] = pval[1:][:, P_t]
             Uc[:-1, an, an] = nval[:-1][:, N_t]
 
-        def inv_into(lines):
-            W, info = torch.linalg.inv_ex(D[lines])
-            if bool((info != 0).any()):
-                raise RuntimeError("A - n0 B is singular on a line: move n0 off the eigenvalue")
-            D[lines] = W
+        # the blocks of a level's lines are inverted in place (FDTD_mode_invert);
+        # host tensors (tests) and blocks whose panels do not fit in shared memory
+        # go through torch
+        infos = []
+        work = int(libFDTD.FDTD_mode_invert_work(nb, NL)) if dev.type == "cuda" else 0
+        if work:
+            work_t = torch.empty(work, dtype=torch.uint8, device=dev)
+            stream = torch.cuda.current_stream(dev).cuda_stream
+
+        def inv_into(lines, lines32):
+            if work:
+                info = torch.empty(len(lines), dtype=torch.int32, device=dev)
+                _check(libFDTD.FDTD_mode_invert(nb, self.device, stream, _ptr(D), _ptr(lines32), len(lines),
+                                                _ptr(work_t), work, _ptr(info)), "FDTD_mode_invert")
+            else:
+                D[lines], info = torch.linalg.inv_ex(D[lines])
+            infos.append(info)
 
         levels = []
         act = list(range(NL))
@@ -213,7 +233,7 @@ class ModeFullVector:
                    "Lc_e1": Lc[lt(e1)].clone(), "Uc_e2": Uc[lt(e2)].clone(),
                    "prev32": i32(even[:len(odd)]), "Lc_odd": Lc[lt(odd)].clone(),
                    "odd_n32": i32(odd_n), "next32": i32(nxt), "Uc_odd_n": Uc[lt(odd_n)].clone()}
-            inv_into(lev["odd"])
+            inv_into(lev["odd"], lev["odd32"])
             newLc = newUc = None
             # the corrections land on distinct (line, row, column) entries, so
             # a gather, a subtraction and a scatter apply them (no sort)
@@ -237,7 +257,9 @@ class ModeFullVector:
             levels.append(lev)
             act = even
         self._top = torch.as_tensor(act, dtype=torch.int32, device=dev)
-        inv_into(lt(act))
+        inv_into(lt(act), self._top)
+        if bool((torch.cat(infos) != 0).any()):
+            raise RuntimeError("A - n0 B is singular on a line: move n0 off the eigenvalue")
         self._W, self._levels = D, levels
         self._P, self._Nr, self._Qp, self._Qn = P_t, N_t, Qp_t, Qn_t
         self._P32, self._N32, self._Qp32, self._Qn32 = (t.to(torch.int32) for t in (P_t, N_t, Qp_t, Qn_t))
