@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(256) k_lines_gemv(int nb, const double* W, con
 // A' the matrix after the panel's row exchanges and G the panel after the
 // elimination of its B columns over all rows (G_K = A'_KK^-1, G_i = -A'_iK G_K),
 // every other column j becomes A_ij = (i in K ? 0 : A'_ij) + G_i A'_Kj.  Three
-// kernels per panel: the panel in shared memory, one CTA per matrix (a serial
+// kernels per panel: the panel in registers, one CTA per matrix (a serial
 // chain of B pivot steps, the bound where a level holds few lines); the row
 // exchanges of the other columns, which also take out A'_K; the update, a rank-B
 // product per 64 x 64 tile (the bound of the first levels: it reads and writes
@@ -285,80 +285,109 @@ __device__ __forceinline__ C2 recip(C2 z) {
     return {r / d, -1.0 / d};
 }
 
-template <int B>
-__global__ void __launch_bounds__(1024) k_inv_panel(int n, double* W, const int* lines, int k0, int* piv,
-                                                    Moves<B>* moves, int* info) {
-    extern __shared__ double2 P[];                    // n rows of B + 1: rows 16 (B + 1) bytes apart, no bank conflicts
+// A thread keeps RP rows of the panel (thread, thread + 640, ...) in registers;
+// only the pivot row and the row it changes places with pass through shared
+// memory.  (With the panel in shared memory, one row per thread, a 606-row panel
+// took 111 us: every column reads and writes all of it.)
+constexpr int kPanelThreads = 640;
+template <int B, int RP>
+__global__ void __launch_bounds__(kPanelThreads, 1) k_inv_panel(int n, double* W, const int* lines, int k0, int* piv,
+                                                                Moves<B>* moves, int* info) {
     __shared__ double best[32];
     __shared__ int where[32];
-    const int z = blockIdx.x, b = min(B, n - k0);
-    double2* A = reinterpret_cast<double2*>(W) + (long long)lines[z] * n * n;
+    __shared__ double2 prow[B], krow[B];
+    const int z = blockIdx.x, b = min(B, n - k0), lane = threadIdx.x & 31;
+    double2* A = reinterpret_cast<double2*>(W) + (long long)lines[z] * n * n + k0;
     int* pv = piv + (long long)z * n;
-    for (int t = threadIdx.x; t < n * b; t += blockDim.x) {
-        const int r = t / b, c = t - r * b;
-        P[r * (B + 1) + c] = A[(long long)r * n + k0 + c];
+    double2 P[RP][B];
+#pragma unroll
+    for (int e = 0; e < RP; e++) {
+        const int r = threadIdx.x + e * kPanelThreads;
+#pragma unroll
+        for (int q = 0; q < B; q++) P[e][q] = r < n && q < b ? A[(long long)r * n + q] : make_double2(0.0, 0.0);
     }
+    if (threadIdx.x < 32) best[threadIdx.x] = -2.0;
     __syncthreads();
+    // P[e][0] is the column at hand: the update shifts the row down by one and
+    // puts the finished column at its end, so the loop body is one copy (fully
+    // unrolled it is 16 times the code, fetched once each: 70 us a panel)
+#pragma unroll 1
     for (int c = 0; c < b; c++) {
         const int k = k0 + c;
         double m = -1.0;
         int at = k;
-        for (int r = threadIdx.x; r < n; r += blockDim.x) {
-            if (r < k) continue;
-            const double2 v = P[r * (B + 1) + c];
-            const double a = fabs(v.x) + fabs(v.y);
-            if (a > m) { m = a; at = r; }
+#pragma unroll
+        for (int e = 0; e < RP; e++) {
+            const int r = threadIdx.x + e * kPanelThreads;
+            const double v = fabs(P[e][0].x) + fabs(P[e][0].y);
+            if (r >= k && r < n && v > m) { m = v; at = r; }
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            const double m2 = __shfl_xor_sync(0xffffffffu, m, o);
-            const int a2 = __shfl_xor_sync(0xffffffffu, at, o);
-            if (m2 > m || (m2 == m && a2 < at)) { m = m2; at = a2; }
-        }
-        if ((threadIdx.x & 31) == 0) { best[threadIdx.x >> 5] = m; where[threadIdx.x >> 5] = at; }
+        auto reduce = [&]() {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const double m2 = __shfl_xor_sync(0xffffffffu, m, o);
+                const int a2 = __shfl_xor_sync(0xffffffffu, at, o);
+                if (m2 > m || (m2 == m && a2 < at)) { m = m2; at = a2; }
+            }
+        };
+        reduce();
+        if (lane == 0) { best[threadIdx.x >> 5] = m; where[threadIdx.x >> 5] = at; }
         __syncthreads();
-        m = best[0];
-        at = where[0];
-        for (int q = 1; q < (int)(blockDim.x >> 5); q++)
-            if (best[q] > m || (best[q] == m && where[q] < at)) { m = best[q]; at = where[q]; }
+        m = best[lane];
+        at = m >= -1.0 ? where[lane] : k;
+        reduce();
         if (threadIdx.x == 0) {
             pv[k] = at;
             if (!(m > 0.0) || isinf(m)) info[z] = 1;
         }
-        // exchange rows k and at, then the pivot row times 1 / pivot (its own
-        // column becomes 1 / pivot)
-        if ((int)threadIdx.x < 32) {
-            const int q = threadIdx.x;
-            double2 x = make_double2(0, 0), y = x;
-            if (q < b) { x = P[k * (B + 1) + q]; y = P[at * (B + 1) + q]; }
-            C2 d = {__shfl_sync(0xffffffffu, y.x, c), __shfl_sync(0xffffffffu, y.y, c)};
-            d = recip(d);
-            if (q < b) {
-                if (at != k) P[at * (B + 1) + q] = x;
-                const C2 v = q == c ? d : d * C2{y.x, y.y};
-                P[k * (B + 1) + q] = make_double2(v.x, v.y);
-            }
-        }
-        __syncthreads();
-        for (int r = threadIdx.x; r < n; r += blockDim.x) {
-            if (r == k) continue;
-            double2* row = P + r * (B + 1);
-            const double2 f = row[c];
+#pragma unroll
+        for (int e = 0; e < RP; e++) {
+            const int r = threadIdx.x + e * kPanelThreads;
 #pragma unroll
             for (int q = 0; q < B; q++) {
-                if (q >= b) break;
-                const double2 u = P[k * (B + 1) + q];
-                double2 a = q == c ? make_double2(0.0, 0.0) : row[q];
-                a.x = fma(-f.x, u.x, fma(f.y, u.y, a.x));
-                a.y = fma(-f.x, u.y, fma(-f.y, u.x, a.y));
-                row[q] = a;
+                if (r == at) prow[q] = P[e][q];
+                if (r == k) krow[q] = P[e][q];
             }
         }
         __syncthreads();
+        const C2 d = recip({prow[0].x, prow[0].y});
+#pragma unroll
+        for (int e = 0; e < RP; e++) {
+            const int r = threadIdx.x + e * kPanelThreads;
+            if (r == k) {
+                // the pivot row times 1 / pivot, 1 / pivot in its own column
+#pragma unroll
+                for (int q = 1; q < B; q++) {
+                    const C2 v = d * C2{prow[q].x, prow[q].y};
+                    P[e][q - 1] = make_double2(v.x, v.y);
+                }
+                P[e][B - 1] = make_double2(d.x, d.y);
+                continue;
+            }
+            if (r == at) {
+#pragma unroll
+                for (int q = 0; q < B; q++) P[e][q] = krow[q];
+            }
+            const C2 f = C2{P[e][0].x, P[e][0].y} * d;
+#pragma unroll
+            for (int q = 1; q < B; q++) {
+                const double2 u = prow[q], a = P[e][q];
+                P[e][q - 1].x = fma(-f.x, u.x, fma(f.y, u.y, a.x));
+                P[e][q - 1].y = fma(-f.x, u.y, fma(-f.y, u.x, a.y));
+            }
+            P[e][B - 1] = make_double2(-f.x, -f.y);
+        }
     }
-    for (int t = threadIdx.x; t < n * b; t += blockDim.x) {
-        const int r = t / b, c = t - r * b;
-        A[(long long)r * n + k0 + c] = P[r * (B + 1) + c];
+#pragma unroll
+    for (int e = 0; e < RP; e++) {
+        const int r = threadIdx.x + e * kPanelThreads;
+#pragma unroll
+        for (int q = 0; q < B; q++) {
+            const int c = b == B ? q : (q + b) % B;      // after b shifts
+            if (r < n && c < b) A[(long long)r * n + c] = P[e][q];
+        }
     }
+    __syncthreads();
     if (threadIdx.x == 0) {
         // where each moved row's content comes from
         Moves<B>& M = moves[z];
@@ -471,17 +500,13 @@ __global__ void __launch_bounds__(256) k_inv_columns(int n, double* W, const int
     for (int j = threadIdx.x; j < n; j += blockDim.x) A[j] = row[pm[j]];
 }
 
-constexpr size_t kInvSmem = 225 * 1024;              // shared memory of the panel kernel
-template <int B>
-size_t panel_bytes(int n) { return sizeof(double2) * (size_t)n * (B + 1); }
-
 // Work memory of the inverses of nl matrices: R, the moves, pivots, permutation.
 size_t inv_work(int n, int nl) {
     auto up = [](size_t x) { return (x + 255) / 256 * 256; };
     return up(sizeof(double2) * 16 * (size_t)n * nl) + up(sizeof(Moves<16>) * (size_t)nl) + 2 * up(sizeof(int) * (size_t)n * nl);
 }
 
-template <int B>
+template <int B, int RP>
 cudaError_t invert(int n, double* W, const int* lines, int nl, unsigned char* work, int* info, cudaStream_t st) {
     auto up = [](size_t x) { return (x + 255) / 256 * 256; };
     double2* R = reinterpret_cast<double2*>(work);
@@ -489,11 +514,9 @@ cudaError_t invert(int n, double* W, const int* lines, int nl, unsigned char* wo
     int* piv = reinterpret_cast<int*>(reinterpret_cast<unsigned char*>(mv) + up(sizeof(Moves<16>) * (size_t)nl));
     int* perm = reinterpret_cast<int*>(reinterpret_cast<unsigned char*>(piv) + up(sizeof(int) * (size_t)n * nl));
     cudaError_t e = cudaMemsetAsync(info, 0, sizeof(int) * nl, st);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_inv_panel<B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInvSmem);
-    const int threads = std::min(1024, (n + 31) / 32 * 32), tiles = (n + 63) / 64;
+    const int threads = std::min(kPanelThreads, (n + 31) / 32 * 32), tiles = (n + 63) / 64;
     for (int k0 = 0; k0 < n && e == cudaSuccess; k0 += B) {
-        k_inv_panel<B><<<nl, threads, panel_bytes<B>(n), st>>>(n, W, lines, k0, piv, mv, info);
+        k_inv_panel<B, RP><<<nl, threads, 0, st>>>(n, W, lines, k0, piv, mv, info);
         if (n > B) {
             k_inv_swap<B><<<dim3((n + 127) / 128, nl), 128, 0, st>>>(n, W, lines, k0, mv, R);
             k_inv_update<B><<<dim3(tiles, tiles, nl), 256, 0, st>>>(n, W, lines, k0, R);
@@ -661,8 +684,7 @@ int FDTD_mode_lines_gemv(int nb, int device, void* stream, const double* W, cons
 }
 
 long long FDTD_mode_invert_work(int nb, int nlines) {
-    // columns per panel: as many as keep a panel in shared memory
-    if (nb < 1 || nlines < 1 || nlines > 65535 || panel_bytes<8>(nb) > kInvSmem) return 0;
+    if (nb < 1 || nlines < 1 || nlines > 65535 || nb > 4 * kPanelThreads) return 0;
     return (long long)inv_work(nb, nlines);
 }
 
@@ -674,9 +696,11 @@ int FDTD_mode_invert(int nb, int device, void* stream, double* W, const int* lin
     MCK(cudaSetDevice(device), "FDTD_mode_invert");
     unsigned char* w = (unsigned char*)work;
     cudaStream_t st = (cudaStream_t)stream;
-    MCK(panel_bytes<16>(nb) <= kInvSmem ? invert<16>(nb, W, lines, nlines, w, info, st)
-                                        : invert<8>(nb, W, lines, nlines, w, info, st),
-        "FDTD_mode_invert");
+    // 64 registers of panel a thread: fewer columns where a thread holds more rows
+    const cudaError_t e = nb <= kPanelThreads       ? invert<16, 1>(nb, W, lines, nlines, w, info, st)
+                          : nb <= 2 * kPanelThreads ? invert<8, 2>(nb, W, lines, nlines, w, info, st)
+                                                    : invert<4, 4>(nb, W, lines, nlines, w, info, st);
+    MCK(e, "FDTD_mode_invert");
     return FDTD_OK;
 }
 

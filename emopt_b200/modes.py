@@ -202,8 +202,7 @@ class ModeFullVector:
             Uc[:-1, an, an] = nval[:-1][:, N_t]
 
         # the blocks of a level's lines are inverted in place (FDTD_mode_invert);
-        # host tensors (tests) and blocks whose panels do not fit in shared memory
-        # go through torch
+        # host tensors (tests) and blocks of more than 2560 rows go through torch
         infos = []
         work = int(libFDTD.FDTD_mode_invert_work(nb, NL)) if dev.type == "cuda" else 0
         if work:

@@ -1,6 +1,6 @@
 """The batched in-place inverses of the mode solver's line blocks
-(FDTD_mode_invert) against numpy: sizes around the panel (16, 8 columns for
-blocks whose 16-column panels do not fit in shared memory) and the 64 x 64 tile,
+(FDTD_mode_invert) against numpy: sizes around the panel (16 columns, 8 or
+4 for blocks of more than 640 or 1280 rows) and the 64 x 64 tile,
 a permutation (every pivot off the diagonal), lines in any order with untouched
 ones between, and singular blocks.
 
@@ -35,7 +35,7 @@ def _invert(W, lines):
     return d.cpu().numpy(), info.cpu().numpy()
 
 
-@pytest.mark.parametrize("nb", [1, 2, 6, 15, 16, 17, 33, 64, 65, 130, 606, 900])
+@pytest.mark.parametrize("nb", [1, 2, 6, 15, 16, 17, 33, 64, 65, 130, 606, 641, 900, 1290])
 def test_inverse_of_random_blocks(nb):
     rng = np.random.default_rng(nb)
     n = 5 if nb < 600 else 2
