@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1) k_inv_panel(int n, double* W
                                                                 Moves<B>* moves, int* info) {
     __shared__ double best[32];
     __shared__ int where[32];
-    __shared__ double2 prow[B], krow[B];
+    __shared__ double2 prow[B], krow[B], dsh;
     const int z = blockIdx.x, b = min(B, n - k0), lane = threadIdx.x & 31;
     double2* A = reinterpret_cast<double2*>(W) + (long long)lines[z] * n * n + k0;
     int* pv = piv + (long long)z * n;
@@ -348,9 +348,15 @@ __global__ void __launch_bounds__(kPanelThreads, 1) k_inv_panel(int n, double* W
                 if (r == at) prow[q] = P[e][q];
                 if (r == k) krow[q] = P[e][q];
             }
+            // one thread divides: done by all, the float64 divisions of 20 warps
+            // took most of a column's time
+            if (r == at) {
+                const C2 v = recip({P[e][0].x, P[e][0].y});
+                dsh = make_double2(v.x, v.y);
+            }
         }
         __syncthreads();
-        const C2 d = recip({prow[0].x, prow[0].y});
+        const C2 d = {dsh.x, dsh.y};
 #pragma unroll
         for (int e = 0; e < RP; e++) {
             const int r = threadIdx.x + e * kPanelThreads;
