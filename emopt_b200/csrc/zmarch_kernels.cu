@@ -173,9 +173,21 @@ struct MarchSmem {
 __device__ __forceinline__ float sfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double sfma(double a, double b, double c) { return __fma_rn(a, b, c); }
 
+// The coefficient pair of one source cell, or zeros.
+__device__ __forceinline__ void pair_load(const float* p, bool in, float& re, float& im) {
+    const float2 v = in ? *reinterpret_cast<const float2*>(p) : make_float2(0, 0);
+    re = v.x; im = v.y;
+}
+__device__ __forceinline__ void pair_load(const double* p, bool in, double& re, double& im) {
+    const double2 v = in ? *reinterpret_cast<const double2*>(p) : make_double2(0, 0);
+    re = v.x; im = v.y;
+}
+
 // Adds (magnetic, sign +) or subtracts (electric) the currents of the sources
 // in `mask` that drive this half step (base 3: M, 0: J) to one vector of cells,
-// in source order.  The coefficients of the next plane are brought to L1.
+// in source order.  Bound by the latency of the coefficients (~350 cycles from
+// L2, on every plane of a march): the pairs of a vector are loaded together,
+// without branches between them, not one cell after the other.
 template <typename T, int BASE>
 __device__ __forceinline__ void vec_sources(const SourceList<T>& src, unsigned mask, int i, int j, int c0, T S, T C,
                                             pk::Vec<T>& a, pk::Vec<T>& b, pk::Vec<T>& c) {
@@ -184,19 +196,19 @@ __device__ __forceinline__ void vec_sources(const SourceList<T>& src, unsigned m
     a.get(f[0]); b.get(f[1]); c.get(f[2]);
     for (; mask; mask &= mask - 1) {
         const DevSource<T>& s = src.s[__ffs(mask) - 1];
-        const int li = i - s.i0, lj = j - s.j0;
+        const int lk = c0 - s.k0;
+        const long long m = 2 * (((long long)(i - s.i0) * s.J + (j - s.j0)) * s.K + lk);
 #pragma unroll
-        for (int e = 0; e < VW; e++) {
-            const int lk = c0 + e - s.k0;
-            if ((unsigned)lk >= (unsigned)s.K) continue;
-            const long long m = 2 * (((long long)li * s.J + lj) * s.K + lk);
+        for (int q = 0; q < 3; q++) {
+            const T* p = s.comp[BASE + q];
+            if (!p) continue;
+            T re[VW], im[VW];
 #pragma unroll
-            for (int q = 0; q < 3; q++) {
-                const T* p = s.comp[BASE + q];
-                if (!p) continue;
-                const T t = sfma(S, ld(p + m), C * ld(p + m + 1));
-                f[q][e] = BASE ? f[q][e] + t : f[q][e] - t;
-                if (li + 1 < s.I) asm volatile("prefetch.global.L1 [%0];" ::"l"(p + m + 2LL * s.J * s.K));
+            for (int e = 0; e < VW; e++) pair_load(p + m + 2 * e, (unsigned)(lk + e) < (unsigned)s.K, re[e], im[e]);
+#pragma unroll
+            for (int e = 0; e < VW; e++) {
+                const T t = sfma(S, re[e], C * im[e]);
+                if ((unsigned)(lk + e) < (unsigned)s.K) f[q][e] = BASE ? f[q][e] + t : f[q][e] - t;
             }
         }
     }
