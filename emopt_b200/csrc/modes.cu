@@ -287,8 +287,9 @@ __device__ __forceinline__ C2 recip(C2 z) {
 
 // A thread keeps RP rows of the panel (thread, thread + 640, ...) in registers;
 // only the pivot row and the row it changes places with pass through shared
-// memory.  (With the panel in shared memory, one row per thread, a 606-row panel
-// took 111 us: every column reads and writes all of it.)
+// memory.  A 606-row panel takes 62 us, one dependent round per column.  (With
+// the panel in shared memory, one row per thread, it took 111 us: every column
+// reads and writes all of it; 67 us with every thread dividing for itself.)
 constexpr int kPanelThreads = 640;
 template <int B, int RP>
 __global__ void __launch_bounds__(kPanelThreads, 1) k_inv_panel(int n, double* W, const int* lines, int k0, int* piv,

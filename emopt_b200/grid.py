@@ -8,7 +8,7 @@ cell wholly inside takes the circle's value, a cut cell gets none of it),
 stacked along z by ``StructuredMaterial3D.add_primitive(prim, z1, z2)``, and
 ``ConstantMaterial3D``.  ``get_values`` returns the Yee-cell averages that the
 reference computes -- area-weighted within a z layer, length-weighted across
-layers -- with one CUDA thread per cell (``FDTD_structured_values``), into a
+layers -- on the GPU, a column of cells per thread (``FDTD_structured_values``), into a
 numpy array or, with ``device=``, into a torch tensor that stays on the GPU
 (``FDTD.set_material_arrays`` takes either).
 

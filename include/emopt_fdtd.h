@@ -111,9 +111,9 @@ int FDTD_last_error(FDTDHandle *h, char *buf, int buflen);
  * device).  Must precede the first call that touches the device. */
 int FDTD_set_device(FDTDHandle *h, int device);
 
-/* Planes per z chunk of the fused time step (kernel 3; 0 = chosen for about
- * 32 resident warps per SM, the default).  A tuning knob; results do not
- * depend on it. */
+/* Planes per z chunk of the fused time step (kernel 3; 0, the default: chunks
+ * of eight planes on average, shorter where a tile's planes cost more).  A
+ * tuning knob; results do not depend on it. */
 int FDTD_set_zchunk(FDTDHandle *h, int planes);
 
 /* Storage/arithmetic precision of FDTD_solve_cw: 64 (default, the reference's
@@ -121,14 +121,17 @@ int FDTD_set_zchunk(FDTDHandle *h, int planes);
  * steady-state fit, probes and outputs stay float64).  Returns a status. */
 int FDTD_set_precision(FDTDHandle *h, int bits);
 
-/* Time-stepping kernel of FDTD_solve_cw: 0 = automatic (default: 6 in
- * float32 when at least 60% of the 64-cell warp tasks lie in no CPML slab,
- * else 5), 1 = H and E kernels with one cell per thread, 3 = one fused H+E
- * kernel per time step whose warps march up z chunks (reads one field/CPML
- * set, writes the other), 5 = H and E kernels with one 2-element vector of x
- * cells per thread, 6 = the kernels of 5 split per half step into an
- * interior launch (tasks in no CPML slab) and a rim launch.  Other values
- * fail with FDTD_ERR_ARG.  Periodic boundaries always use 1. */
+/* Time-stepping kernel of FDTD_solve_cw: 0 = automatic (default: 3 where
+ * rows hold more than 16 vectors of 16 bytes, no axis is periodic and the
+ * second set of fields fits in memory; else 6 in float32 when at least 60% of
+ * the 64-cell warp tasks lie in no CPML slab; else 5), 1 = H and E kernels
+ * with one cell per thread, 3 = one fused H+E kernel per time step whose
+ * CTAs march up z chunks (reads one field/CPML set, writes the other), 5 = H
+ * and E kernels with one 2-element vector of x cells per thread, 6 = the
+ * kernels of 5 split per half step into an interior launch (tasks in no CPML
+ * slab) and a rim launch.  3, 5 and 6 give the same bits where auto chooses
+ * among them.  Other values fail with FDTD_ERR_ARG.  Periodic boundaries
+ * always use 1. */
 int FDTD_set_kernel(FDTDHandle *h, int which);
 
 /* Page-locks (cudaHostRegister, portable) / releases host memory that is
