@@ -39,6 +39,13 @@ __global__ void k_material_coeffs(const c128* eps, const c128* mu, int Nx, int N
     if (mu) bH_out[p] = T(dt / mu[g].real);
 }
 
+template <typename T>
+__global__ void k_fill(T* a, long long n, T v) {
+    for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < n;
+         g += (long long)gridDim.x * blockDim.x)
+        a[g] = v;
+}
+
 __global__ void k_uniform_check(const c128* mu, long long n, int* flag) {
     double ref = mu[0].real;
     for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < n;
@@ -141,6 +148,11 @@ void launch_material_coeffs(const c128* eps, const c128* mu, int Nx, int Ny, int
                                                              b_out, a_out, bH_out);
 }
 
+template <typename T>
+void launch_fill(T* a, long long n, T v, cudaStream_t st) {
+    k_fill<T><<<1184, 256, 0, st>>>(a, n, v);
+}
+
 void launch_uniform_check(const c128* mu, long long n, int* flag, cudaStream_t st) {
     k_uniform_check<<<296, 256, 0, st>>>(mu, n, flag);
 }
@@ -187,6 +199,7 @@ void launch_probe(const T* Ex, const T* Ey, const T* Ez, ProbeDev pd, long long*
 }
 
 #define INST(T)                                                                                 \
+    template void launch_fill<T>(T*, long long, T, cudaStream_t);                               \
     template void launch_material_coeffs<T>(const c128*, const c128*, int, int, int, int,       \
                                             double, bool, T*, T*, T*, cudaStream_t);            \
     template void launch_source_coeffs<T>(const c128*, int, int, int, int, int, int, const T*,   \

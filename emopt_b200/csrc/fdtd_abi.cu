@@ -70,6 +70,7 @@ struct Resident {
     DevBuf F[2][6];          // fields Ex Ey Ez Hx Hy Hz; set 1: the fused step's second set
     DevBuf bE[3], aE[3], bH[3];
     bool mu_uniform[3] = {true, true, true};
+    bool mu_arrays = false;  // some component varies: bH holds all three
     double mu_value[3] = {1, 1, 1};
     bool lossy = false;
     bool coeffs_valid = false;
@@ -908,6 +909,15 @@ int prepare_materials(FDTDHandle* h, Resident<T>& r) {
             CK(cudaGetLastError());
         }
     }
+    // the vector kernels read dt/mu of all three components or of none, so a
+    // uniform component beside a varying one gets an array as well
+    r.mu_arrays = !(r.mu_uniform[0] && r.mu_uniform[1] && r.mu_uniform[2]);
+    for (int c = 0; c < 3 && r.mu_arrays; c++) {
+        if (!r.mu_uniform[c]) continue;
+        CK(r.bH[c].ensure(sizeof(T) * cells));
+        fdtdb::launch_fill<T>(dptr<T>(r.bH[c]), (long long)cells, T(h->dt / r.mu_value[c]), h->stream);
+        CK(cudaGetLastError());
+    }
     // CPML tables reordered by local slab index (min slab reversed) with 1/kappa,
     // and the forms the fused step reads (MarchArgs); one upload for all of them
     using Dup = typename fdtdb::pk::DupOf<T>::type;
@@ -1029,7 +1039,7 @@ fdtdb::GridView<T> make_view(FDTDHandle* h, Resident<T>& r, int set = 0) {
     for (int c = 0; c < 3; c++) {
         g.bE[c] = dptr<T>(r.bE[c]);
         g.aE[c] = h->lossy ? dptr<T>(r.aE[c]) : nullptr;
-        g.bHarr[c] = r.mu_uniform[c] ? nullptr : dptr<T>(r.bH[c]);
+        g.bHarr[c] = r.mu_arrays ? dptr<T>(r.bH[c]) : nullptr;
         g.bH[c] = T(h->dt / r.mu_value[c]);
         g.bc[c] = h->bc[c];
     }

@@ -64,7 +64,7 @@ struct GridView {
     T odx, ody, odz;
     const T* bE[3];                // E update: b = dt/eps (or the lossy form)
     const T* aE[3];                // lossy E update: a (null when lossless)
-    const T* bHarr[3];             // H update: dt/mu per cell (null when uniform)
+    const T* bHarr[3];             // H update: dt/mu per cell (all three, or null when all are uniform)
     T bH[3];                       // uniform dt/mu
     char bc[3];
     // a neighbouring z slab holds the plane below local index 0 (zlo) or above

@@ -94,6 +94,10 @@ void launch_material_coeffs(const c128* eps_or_null, const c128* mu_or_null, int
                             int Nz, int px, double dt, bool lossy, T* b_out, T* a_out_or_null,
                             T* bH_out, cudaStream_t st);
 
+// a[0 .. n - 1] = v.
+template <typename T>
+void launch_fill(T* a, long long n, T v, cudaStream_t st);
+
 // Returns (on the device) 1 in *flag when every mu[c].real equals mu[0].real.
 void launch_uniform_check(const c128* mu, long long n, int* flag, cudaStream_t st);
 
