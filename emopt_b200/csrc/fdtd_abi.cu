@@ -67,6 +67,7 @@ template <typename T>
 struct Resident {
     int Nx = 0, Ny = 0, Nz = 0, px = 0;
     DevBuf arena;            // the one allocation that alloc_resident cuts into the arrays
+    DevBuf second;           // ... and alloc_second into set 1 of F and psi
     DevBuf F[2][6];          // fields Ex Ey Ez Hx Hy Hz; set 1: the fused step's second set
     DevBuf bE[3], aE[3], bH[3];
     bool mu_uniform[3] = {true, true, true};
@@ -86,6 +87,11 @@ struct Resident {
     int halo = 0;            // planes of halo below and above the fields (z slabs)
     DevBuf psamp;            // z slab: probe samples of all slabs [3][npoints]
 
+    void release_second() {
+        for (auto& b : F[1]) b.release();
+        for (auto& a : psi[1]) for (auto& b : a) b.release();
+        second.release();
+    }
     void release_all() {
         for (auto& s : F) for (auto& b : s) b.release();
         for (int c = 0; c < 3; c++) { bE[c].release(); aE[c].release(); bH[c].release(); }
@@ -102,6 +108,7 @@ struct Resident {
         steptab.release(); stepbase.release(); flag.release(); err.release();
         pwin.release(); pA.release(); pphi.release(); ptimes.release(); pout.release(); pmap.release();
         psamp.release();
+        release_second();
         arena.release();
         coeffs_valid = false;
         Nx = Ny = Nz = px = 0;
@@ -816,28 +823,42 @@ bool march_possible(const FDTDHandle* h) {
            h->Nz * ((h->w[2] + h->w[3]) * px) < lim && (h->w[4] + h->w[5]) * (h->Ny * px) < lim;
 }
 
-// Allocates the resident arrays for the current grid and PML widths.
-// march: the arrays of the fused step (a second set of the fields and of the
-// H-update CPML state, whole-vector x-slab rows).
+// Cuts one allocation into arrays of the given sizes: allocating and freeing the
+// ~35 arrays of a served request one by one cost about 10 ms each way.
+struct Want { DevBuf* b; size_t bytes; };
+
+cudaError_t cut(DevBuf& from, const std::vector<Want>& want) {
+    auto up = [](size_t n) { return (n + 511) / 512 * 512; };
+    size_t total = 0, at = 0;
+    for (const Want& w : want) total += up(w.bytes);
+    const cudaError_t e = from.ensure(total);
+    if (e != cudaSuccess) return e;
+    for (const Want& w : want) {
+        w.b->p = (unsigned char*)from.p + at;
+        w.b->bytes = w.bytes;
+        w.b->owned = false;
+        at += up(w.bytes);
+    }
+    return cudaSuccess;
+}
+
+// Allocates the resident arrays for the current grid and PML widths, but for the
+// fused step's second set (alloc_second).
+// x_rows: slots in a row of the x-slab state.
 // halo = 1 (z slabs): the six field arrays get one plane below and one above
 // the slab; the interior starts one plane into each array.
 template <typename T>
-int alloc_resident(FDTDHandle* h, Resident<T>& r, bool march, int halo = 0) {
+int alloc_resident(FDTDHandle* h, Resident<T>& r, int x_rows, int halo = 0) {
     int px = (h->Nx + 31) / 32 * 32;
     size_t cells = (size_t)h->Nz * h->Ny * px;
     size_t fcells = (size_t)(h->Nz + 2 * halo) * h->Ny * px;
-    long long slab[3] = {(long long)h->Nz * h->Ny * (march ? x_slab<T>(h).pitch : h->w[0] + h->w[1]),
+    long long slab[3] = {(long long)h->Nz * h->Ny * x_rows,
                          (long long)h->Nz * (h->w[2] + h->w[3]) * px,
                          (long long)(h->w[4] + h->w[5]) * h->Ny * px};
-    // One allocation holds all of them: allocating and freeing the ~35 arrays of
-    // a served request one by one cost about 10 ms each way.
-    struct Want { DevBuf* b; size_t bytes; };
     std::vector<Want> want;
-    for (int s = 0; s < (march ? 2 : 1); s++) {
-        for (int c = 0; c < 6; c++) want.push_back({&r.F[s][c], sizeof(T) * fcells});
-        for (int a = 0; a < 3; a++)
-            for (int q = 0; q < (s ? 2 : 4); q++) want.push_back({&r.psi[s][a][q], sizeof(T) * (size_t)(slab[a] ? slab[a] : 1)});
-    }
+    for (int c = 0; c < 6; c++) want.push_back({&r.F[0][c], sizeof(T) * fcells});
+    for (int a = 0; a < 3; a++)
+        for (int q = 0; q < 4; q++) want.push_back({&r.psi[0][a][q], sizeof(T) * (size_t)(slab[a] ? slab[a] : 1)});
     for (int c = 0; c < 3; c++) want.push_back({&r.bE[c], sizeof(T) * cells});
     for (int s = 0; s < 2; s++)
         for (int c = 0; c < 6; c++) want.push_back({&r.snap[s][c], sizeof(T) * cells});
@@ -845,25 +866,26 @@ int alloc_resident(FDTDHandle* h, Resident<T>& r, bool march, int halo = 0) {
     want.push_back({&r.stepbase, sizeof(long long)});
     want.push_back({&r.flag, sizeof(int) * 4});
     want.push_back({&r.err, sizeof(int) * 4});
-    auto up = [](size_t n) { return (n + 511) / 512 * 512; };
-    size_t total = 0;
     bool same = r.Nx == h->Nx && r.Ny == h->Ny && r.Nz == h->Nz && r.px == px && r.halo == halo;
-    for (const Want& w : want) {
-        total += up(w.bytes);
-        same = same && w.b->p && w.b->bytes >= w.bytes;
-    }
+    for (const Want& w : want) same = same && w.b->p && w.b->bytes >= w.bytes;
     if (same) return FDTD_OK;
     r.release_all();
-    CK(r.arena.ensure(total));
+    CK(cut(r.arena, want));
     r.Nx = h->Nx; r.Ny = h->Ny; r.Nz = h->Nz; r.px = px; r.halo = halo;
-    size_t at = 0;
-    for (const Want& w : want) {
-        w.b->p = (unsigned char*)r.arena.p + at;
-        w.b->bytes = w.bytes;
-        w.b->owned = false;
-        at += up(w.bytes);
-    }
     return FDTD_OK;
+}
+
+// The second set of the fields and of the H-update CPML state, which the fused
+// step alternates with the first.  It is an allocation of its own: adding it or
+// giving it up leaves the other arrays and the coefficients as they are.
+template <typename T>
+cudaError_t alloc_second(Resident<T>& r) {
+    if (r.second.p) return cudaSuccess;
+    std::vector<Want> want;
+    for (int c = 0; c < 6; c++) want.push_back({&r.F[1][c], r.F[0][c].bytes});
+    for (int a = 0; a < 3; a++)
+        for (int q = 0; q < 2; q++) want.push_back({&r.psi[1][a][q], r.psi[0][a][q].bytes});
+    return cut(r.second, want);
 }
 
 // Material upload (one component at a time through one staging buffer) and
@@ -871,6 +893,7 @@ int alloc_resident(FDTDHandle* h, Resident<T>& r, bool march, int halo = 0) {
 template <typename T>
 int prepare_materials(FDTDHandle* h, Resident<T>& r) {
     ensure_tables(h);
+    r.coeffs_valid = false;      // until all of them are made
     long long n = (long long)h->Nx * h->Ny * h->Nz;
     size_t cells = (size_t)h->Nz * h->Ny * r.px;
     CK(r.stage.ensure(sizeof(c128) * n));
@@ -1172,34 +1195,65 @@ int solve_impl(FDTDHandle* h, const FDTDSolveOptions* o, FDTDSolveResult* res) {
     else if (kid == 3 && !march_possible<T>(h)) kid = pair;
     int rc;
     CK(cudaEventRecord(h->ev[2], h->stream));
-    rc = alloc_resident<T>(h, r, kid == 3);
-    if (rc != FDTD_OK && kid == 3 && h->kernel == 0) {
-        // no room for the second field set: the pair updates in place
-        cudaGetLastError();
-        r.release_all();
-        kid = pair;
-        rc = alloc_resident<T>(h, r, false);
-    }
-    if (rc != FDTD_OK) return rc;
-    const bool fused = kid == 3;
-    const bool vec = kid == 5;
-    const bool split = kid == 6;
-    CK(cudaMemsetAsync(r.err.p, 0, sizeof(int) * 4, h->stream));
-    if (!o->materials_unchanged || !r.coeffs_valid) {
-        if ((rc = prepare_materials<T>(h, r)) != FDTD_OK) return rc;
-        launches += 3 + 3 + 3;   // eps coefficients, uniform checks, mu coefficients (upper bound)
-    }
-    fdtdb::SourceList<T> src;
-    if ((rc = prepare_sources<T>(h, r, src)) != FDTD_OK) return rc;
-    for (int q = 0; q < src.n; q++)
-        for (int c = 0; c < 6; c++) launches += src.s[q].comp[c] ? 1 : 0;
-
     const long long Tn = o->Tn;
     const bool fixed = o->fixed_steps > 0;
     long long last = fixed ? o->fixed_steps - 1 : (long long)floor(o->Nmax);
     if (!fixed && o->Nmax < 0) last = -1;
-    long long max_steps = (last + 1 > 0 ? last + 1 : 0) + 2 * Tn + Tn + 1;
-    CK(r.steptab.ensure(sizeof(double4) * max_steps));
+    const long long max_steps = (last + 1 > 0 ? last + 1 : 0) + 2 * Tn + Tn + 1;
+    const int nconv = o->nconv > 0 ? o->nconv : 0, nc = nconv > 0 ? nconv : 1;
+    // x-slab rows that serve either layout of that state
+    const XSlab xs = x_slab<T>(h);
+    const int x_rows = std::max(h->w[0] + h->w[1], xs.ok ? xs.pitch : 0);
+    fdtdb::SourceList<T> src;
+    bool materials = !o->materials_unchanged;
+    // everything but the second set of the fused step
+    auto set_up = [&]() -> int {
+        int rc;
+        if ((rc = alloc_resident<T>(h, r, x_rows)) != FDTD_OK) return rc;
+        CK(cudaMemsetAsync(r.err.p, 0, sizeof(int) * 4, h->stream));
+        if (materials || !r.coeffs_valid) {
+            if ((rc = prepare_materials<T>(h, r)) != FDTD_OK) return rc;
+            materials = false;
+            launches += 3 + 3 + 3;   // eps coefficients, uniform checks, mu coefficients (upper bound)
+        }
+        if ((rc = prepare_sources<T>(h, r, src)) != FDTD_OK) return rc;
+        CK(r.steptab.ensure(sizeof(double4) * max_steps));
+        CK(r.pwin.ensure(sizeof(double) * 9 * nc));
+        CK(r.pA.ensure(sizeof(double) * 2 * nc));
+        CK(r.pphi.ensure(sizeof(double) * 2 * nc));
+        CK(r.ptimes.ensure(sizeof(double) * 3));
+        CK(r.pout.ensure(sizeof(double) * 4));
+        CK(r.pmap.ensure(sizeof(long long) * nc));
+        return FDTD_OK;
+    };
+    rc = set_up();
+    if (rc == FDTD_ERR_CUDA && r.second.p) {
+        // the second set of an earlier solve may hold the memory this one needs
+        cudaGetLastError();
+        r.release_second();
+        rc = set_up();
+    }
+    if (rc != FDTD_OK) return rc;
+    std::vector<int4> work;
+    if (kid == 3) {
+        int dev_sms = 148;
+        cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, h->device);
+        fdtdb::march_work<T>(make_view<T>(h, r), dev_sms, h->zchunk, work);
+        cudaError_t e = r.work.ensure(sizeof(int4) * work.size());
+        if (e == cudaSuccess) e = alloc_second<T>(r);
+        if (e != cudaSuccess && h->kernel != 0) return h->cuda_fail(e, "the second field set of the fused step");
+        if (e != cudaSuccess) {
+            // no room for the second field set: the pair updates in place
+            cudaGetLastError();
+            kid = pair;
+            work.clear();
+        }
+    }
+    const bool fused = kid == 3;
+    const bool vec = kid == 5;
+    const bool split = kid == 6;
+    for (int q = 0; q < src.n; q++)
+        for (int c = 0; c < 6; c++) launches += src.s[q].comp[c] ? 1 : 0;
     fdtdb::launch_step_table(dptr<double4>(r.steptab), max_steps, h->dt, h->src_T,
                              h->src_min, h->src_k, h->stream);
     launches++;
@@ -1212,14 +1266,6 @@ int solve_impl(FDTDHandle* h, const FDTDSolveOptions* o, FDTDSolveResult* res) {
                 CK(cudaMemsetAsync(r.psi[s][a][q].p, 0, r.psi[s][a][q].bytes, h->stream));
     }
     // convergence probe state
-    int nconv = o->nconv > 0 ? o->nconv : 0;
-    int nc = nconv > 0 ? nconv : 1;
-    CK(r.pwin.ensure(sizeof(double) * 9 * nc));
-    CK(r.pA.ensure(sizeof(double) * 2 * nc));
-    CK(r.pphi.ensure(sizeof(double) * 2 * nc));
-    CK(r.ptimes.ensure(sizeof(double) * 3));
-    CK(r.pout.ensure(sizeof(double) * 4));
-    CK(r.pmap.ensure(sizeof(long long) * nc));
     CK(cudaMemsetAsync(r.pwin.p, 0, sizeof(double) * 9 * nc, h->stream));
     CK(cudaMemsetAsync(r.pA.p, 0, sizeof(double) * 2 * nc, h->stream));
     CK(cudaMemsetAsync(r.pphi.p, 0, sizeof(double) * 2 * nc, h->stream));
@@ -1251,12 +1297,7 @@ int solve_impl(FDTDHandle* h, const FDTDSolveOptions* o, FDTDSolveResult* res) {
     }
     // field set that holds the state after `steps` time steps
     auto cur_set = [&](long long steps) -> T* const* { return (fused && (steps & 1)) ? f1 : f0; };
-    int dev_sms = 148;
-    cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, h->device);
-    std::vector<int4> work;
     if (fused) {
-        fdtdb::march_work<T>(g0, dev_sms, h->zchunk, work);
-        CK(r.work.ensure(sizeof(int4) * work.size()));
         CK(cudaMemcpyAsync(r.work.p, work.data(), sizeof(int4) * work.size(), cudaMemcpyDefault, h->stream));
         CK(cudaStreamSynchronize(h->stream));
     }

@@ -70,7 +70,7 @@ template <typename T>
 int slab_begin_impl(FDTDHandle* h, const FDTDSolveOptions* o, const long long* cells, int np) {
     Resident<T>& r = resident<T>(h);
     int rc;
-    if ((rc = alloc_resident<T>(h, r, false, 1)) != FDTD_OK) return rc;
+    if ((rc = alloc_resident<T>(h, r, h->w[0] + h->w[1], 1)) != FDTD_OK) return rc;
     CK(cudaMemsetAsync(r.err.p, 0, sizeof(int) * 4, h->stream));
     if (!o->materials_unchanged || !r.coeffs_valid)
         if ((rc = prepare_materials<T>(h, r)) != FDTD_OK) return rc;
