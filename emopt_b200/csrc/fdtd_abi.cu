@@ -1178,19 +1178,24 @@ int solve_impl(FDTDHandle* h, const FDTDSolveOptions* o, FDTDSolveResult* res) {
                        (long long)h->Nz * h->Ny * (h->w[0] + h->w[1]) < (1LL << 31);
     // kernel ids: 0 auto, 1 scalar H/E pair, 3 fused step, 5 vector H/E pair, 6
     // vector pair split into interior and rim launches.  Auto takes the fused
-    // step wherever it is possible but for rows of at most 16 vectors, which
-    // leave half of its lanes idle (56 x 48 x 44 in float32: 12.6 us per step
-    // either way; 72 x 72 x 72: 18.2 against 22.7).  Without it: the split pair in
-    // float32 when at least 60% of the warp tasks lie in no CPML slab (the
-    // 1201 x 601 x 301 grating slab, 69%: 3293 instead of 3605 us per step;
-    // the 321 x 161 x 101 MMI block, 23%: 143 instead of 122), else the
-    // vector pair.  All of them round alike, so the choice changes no bit.
+    // step where it is possible and faster (march_pays), but for rows of at most
+    // 16 vectors, which leave half of its lanes idle (56 x 48 x 44 in float32: 12.6
+    // us per step either way; 72 x 72 x 72: 18.2 against 22.7).  Without it: the
+    // split pair in float32 when at least 60% of the warp tasks lie in no CPML
+    // slab (the 1201 x 601 x 301 grating slab, 69%: 3293 instead of 3605 us per
+    // step; the 321 x 161 x 101 MMI block, 23%: 143 instead of 122), else the
+    // vector pair.  The fused step rounds as the pair that auto would take in its
+    // place (src_general), so that choice changes no bit.
     bool split_rule = false;
     if (sizeof(T) == 4 && !periodic && small_index)
         split_rule = fdtdb::split_interior_fraction<T>(make_view<T>(h, r, 0)) >= 0.6;
     int kid = h->kernel;
     const int pair = periodic || !small_index ? 1 : split_rule ? 6 : 5;
-    if (kid == 0) kid = march_possible<T>(h) && h->Nx > 16 * (16 / (int)sizeof(T)) ? 3 : pair;
+    int dev_sms = 148;
+    cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, h->device);
+    if (kid == 0)
+        kid = march_possible<T>(h) && h->Nx > 16 * (16 / (int)sizeof(T)) &&
+                      fdtdb::march_pays<T>(make_view<T>(h, r), dev_sms, split_rule) ? 3 : pair;
     else if (periodic || !small_index) kid = 1;
     else if (kid == 3 && !march_possible<T>(h)) kid = pair;
     int rc;
@@ -1236,8 +1241,6 @@ int solve_impl(FDTDHandle* h, const FDTDSolveOptions* o, FDTDSolveResult* res) {
     if (rc != FDTD_OK) return rc;
     std::vector<int4> work;
     if (kid == 3) {
-        int dev_sms = 148;
-        cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, h->device);
         fdtdb::march_work<T>(make_view<T>(h, r), dev_sms, h->zchunk, work);
         cudaError_t e = r.work.ensure(sizeof(int4) * work.size());
         if (e == cudaSuccess) e = alloc_second<T>(r);

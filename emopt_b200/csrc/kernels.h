@@ -80,6 +80,11 @@ cudaError_t launch_step_march(const MarchArgs<T>& a, const SourceList<T>& src, c
 template <typename T>
 cudaError_t march_maps(MarchArgs<T>& a);
 
+// Is the fused step faster on this grid (`sms` multiprocessors) than the vector
+// pair, or (split) the split pair?
+template <typename T>
+bool march_pays(const GridView<T>& g, int sms, bool split);
+
 // The work list of the fused step: chunks of zc planes, or (zc = 0) chunks of
 // equal estimated time for `sms` multiprocessors.
 template <typename T>

@@ -681,19 +681,94 @@ cudaError_t launch_step_march(const MarchArgs<T>& a, const SourceList<T>& src, c
               : launch_one<T, false, false>(a, src, work, nwork, step_base, off, st);
 }
 
-// The chunks of the tile columns.  A CTA takes as long as its slowest warp, and
-// CPML state makes planes slow (cycles per plane on the 321 x 161 x 101 grid
-// with 20-cell slabs: 3650 in none, 4600 in an x slab, 5900 z, 6700 y, 8300 in
-// all three), so every column is cut into chunks of equal estimated time, the
-// column with the longest ones first.  Chunks of 8 planes on average, in as many
-// waves as that takes, keep neighbouring tiles close in z (their halo rows hit
-// L2) and the last wave short: 105.6 us a step on that grid against 107.5 with
-// 9-13 planes, 118 in one wave and 125.6 in equal chunks of 26; in float64 185
-// against 227 in one wave.  Grids that fill less than a wave take one wave.
+namespace {
+
+// Estimated cycles (thousands) of a plane of each tile column.  A CTA takes as
+// long as its slowest warp, and CPML state makes planes slow (cycles per plane on
+// the 321 x 161 x 101 grid in float32 with 20-cell slabs: 3650 in none, 4600 in an
+// x slab, 5900 z, 6700 y, 8300 in all three).
+template <typename T>
+struct MarchCost {
+    static constexpr int V = pk::Vec<T>::N, R = kNW - 1;
+    const GridView<T>& g;
+    const int ntx, nty, ncol;
+    std::vector<char> inz;           // planes in a z slab, and their number
+    int nz = 0;
+
+    explicit MarchCost(const GridView<T>& g)
+        : g(g), ntx(x_tiles<T>(g.Nx)), nty((g.Ny + R - 1) / R), ncol(ntx * nty), inz(g.Nz) {
+        for (int i = 0; i < g.Nz; i++) nz += inz[i] = slab_local(g.pml[2], i + g.pml[2].off, true) >= 0;
+    }
+    double plane(int col, bool z) const {
+        const int x = col % ntx, y = col / ntx;
+        const PmlAxis<T>*P = g.pml;
+        const int c0 = x * 30 * V, c1 = std::min(c0 + 32 * V, g.Nx), j0 = std::max(0, y * R - 1), j1 = std::min(y * R + R, g.Ny);
+        const bool sx = c0 < P[0].w0 || (P[0].w1 > 0 && c1 > P[0].edge_max);
+        const bool sy = j0 < P[1].w0 || (P[1].w1 > 0 && j1 > P[1].edge_max);
+        return 3.65 + (sx ? 0.9 : 0.0) + (sy && z ? 3.8 : sy ? 3.0 : z ? 2.2 : 0.0);
+    }
+    double column(int col) const { return nz * plane(col, true) + (g.Nz - nz) * plane(col, false); }
+    // Does the tile hold more x-slab state than a box copy brings (cells of both
+    // slabs, mostly)?
+    bool wide_x(int x) const {
+        const PmlAxis<T>& P = g.pml[0];
+        auto up = [](int k) { return (k + V - 1) / V * V; };
+        const int c0 = x * 30 * V, c1 = std::min(c0 + 32 * V, up(g.Nx));
+        const int first = P.edge_max & ~(V - 1);            // the vector the max slab starts in
+        const int lo = std::min(c1, up(P.w0)) - c0, hi = P.w1 > 0 ? c1 - std::max(c0, first) : 0;
+        return (std::max(lo, 0) + std::max(hi, 0)) * (int)sizeof(T) > (int)kXRow;
+    }
+};
+
+}  // namespace
+
+// Is the fused step faster than the pair that would run in its place (split: the
+// split pair)?  Its time goes with the cycles per CTA slot (t, thousands), the
+// pair's with its warp tasks of 64 cells (q: their number per thousand cycles of
+// the fused step).  A CTA works for seven rows whether they are there or not, and
+// in slab code where one of them lies in a slab, so grids of few rows, or mostly
+// slab, leave the fused step behind once they are too large to be bound by
+// launches and latency.  us per step, pair and fused:
+//   float32  512x1x300 (t 21, q 0.11) 10.6 13.9 (split pair 20.8), 150x2x1008 (31,
+//            0.19) 15.6 19.6, 580x1x947 (65, 0.15) 18.6 33.8 (split 28.0);
+//            256x16x100 (23, 0.27) 16.7 15.1, 59x105x114 (37, 0.33) 24.0 21.9
+//   float64  88x1x486 (15, 0.06) 10.6 12.4, 179x2x791 (29, 0.16) 14.7 17.8,
+//            324x1x1082 (80, 0.08) 16.8 39.4, 126x33x171 (62, 0.18) 30.5 36.2,
+//            374x36x39 (40, 0.21) 22.9 25.8, 119x31x163 (40, 0.25) 27.1 30.0;
+//            128x1x100 (5, 0.04) 10.6 8.1, 128x16x100 (23, 0.14) 16.7 14.7,
+//            305x34x34 (25, 0.23) 19.7 16.8, 101x76x65 (33, 0.30) 26.6 22.2
+// Where a tile's x-slab state does not come by box copies its planes take about
+// a quarter longer in float64: 72x90x90 with 15-cell slabs (51, 0.32) 35.1 40.0,
+// 62x79x136 with 12 (34, 0.32) 27.0 30.7, 93x141x73 with 20 (67, 0.31) 51.5 54.3,
+// but 62x90x90 (26, 0.32) 24.9 21.4.  Over 710 grids of up to 3 M cells the pair's
+// time over the chosen one's is 1.256 in float64 and 1.432 in float32 (geometric
+// mean; the better of both: 1.261, 1.433); near the lines either side wins by up
+// to 8%.
+template <typename T>
+bool march_pays(const GridView<T>& g, int sms, bool split) {
+    const MarchCost<T> c(g);
+    double t = 0.0;
+    for (int q = 0; q < c.ncol; q++) t += c.column(q);
+    t /= kMinB * (sms > 0 ? sms : 148);
+    const double q = 1e-3 * ((g.Nx + 63) / 64) * g.Ny * g.Nz / t;
+    if (sizeof(T) == 4) return t <= (split ? 33.0 : 20.5) || q >= 0.25;
+    bool wide = false;
+    for (int x = 0; x < c.ntx; x++) wide = wide || c.wide_x(x);
+    if (wide && t > 31.0 && q < 0.36) return false;
+    return t <= 13.0 || q >= (t <= 25.0 ? 0.12 : t <= 33.0 ? 0.17 : 0.29);
+}
+
+// The chunks of the tile columns: every column is cut into chunks of equal
+// estimated time (MarchCost), the column with the longest ones first.  Chunks of 8
+// planes on average, in as many waves as that takes, keep neighbouring tiles close
+// in z (their halo rows hit L2) and the last wave short: 105.6 us a step on the
+// 321 x 161 x 101 grid against 107.5 with 9-13 planes, 118 in one wave and 125.6 in
+// equal chunks of 26; in float64 185 against 227 in one wave.  Grids that fill
+// less than a wave take one wave.
 template <typename T>
 void march_work(const GridView<T>& g, int sms, int zc, std::vector<int4>& work) {
-    constexpr int V = pk::Vec<T>::N, R = kNW - 1;
-    const int ntx = x_tiles<T>(g.Nx), nty = (g.Ny + R - 1) / R, Nz = g.Nz;
+    const MarchCost<T> cost(g);
+    const int ntx = cost.ntx, nty = cost.nty, ncol = cost.ncol, Nz = g.Nz;
     work.clear();
     if (zc > 0) {
         for (int i = 0; i < Nz; i += zc)
@@ -701,22 +776,10 @@ void march_work(const GridView<T>& g, int sms, int zc, std::vector<int4>& work) 
                 for (int x = 0; x < ntx; x++) work.push_back(make_int4(x, y, i, std::min(i + zc, Nz)));
         return;
     }
-    const PmlAxis<T>*P = g.pml;
-    std::vector<char> inz(Nz);
-    int nz_slab = 0;
-    for (int i = 0; i < Nz; i++) nz_slab += inz[i] = slab_local(P[2], i + P[2].off, true) >= 0;
-    // estimated cycles (thousands) of a plane of column (x, y), outside and in a z slab
-    auto cost = [&](int x, int y, bool z) {
-        const int c0 = x * 30 * V, c1 = std::min(c0 + 32 * V, g.Nx), j0 = std::max(0, y * R - 1), j1 = std::min(y * R + R, g.Ny);
-        const bool sx = c0 < P[0].w0 || (P[0].w1 > 0 && c1 > P[0].edge_max);
-        const bool sy = j0 < P[1].w0 || (P[1].w1 > 0 && j1 > P[1].edge_max);
-        return 3.65 + (sx ? 0.9 : 0.0) + (sy && z ? 3.8 : sy ? 3.0 : z ? 2.2 : 0.0);
-    };
-    const int ncol = ntx * nty, slots = std::max(1, kMinB * (sms > 0 ? sms : 148));
+    const int slots = std::max(1, kMinB * (sms > 0 ? sms : 148));
     const double fill = 8.0;                       // first copies and the plane before the chunk
     std::vector<double> total(ncol);
-    for (int c = 0; c < ncol; c++)
-        total[c] = nz_slab * cost(c % ntx, c / ntx, true) + (Nz - nz_slab) * cost(c % ntx, c / ntx, false);
+    for (int c = 0; c < ncol; c++) total[c] = cost.column(c);
     // kChunk planes a chunk on average, one wave of CTAs at least; the column with
     // the longest chunks is cut first
     constexpr double kChunk = 8.0;
@@ -734,11 +797,11 @@ void march_work(const GridView<T>& g, int sms, int zc, std::vector<int4>& work) 
     // cut the columns; chunk k of every column before chunk k + 1 of any
     std::vector<std::vector<int4>> rank;
     for (int c = 0; c < ncol; c++) {
-        const double in = cost(c % ntx, c / ntx, true), out = cost(c % ntx, c / ntx, false);
+        const double in = cost.plane(c, true), out = cost.plane(c, false);
         double acc = 0.0;
         int from = 0, k = 1;
         for (int i = 0; i < Nz; i++) {
-            acc += inz[i] ? in : out;
+            acc += cost.inz[i] ? in : out;
             if (i + 1 < Nz && !(k < best[c] && acc >= total[c] * k / best[c])) continue;
             if ((int)rank.size() < k) rank.resize(k);
             rank[k - 1].push_back(make_int4(c % ntx, c / ntx, from, i + 1));
@@ -755,6 +818,8 @@ template cudaError_t launch_step_march<double>(const MarchArgs<double>&, const S
                                                const long long*, int, cudaStream_t);
 template cudaError_t march_maps<float>(MarchArgs<float>&);
 template cudaError_t march_maps<double>(MarchArgs<double>&);
+template bool march_pays<float>(const GridView<float>&, int, bool);
+template bool march_pays<double>(const GridView<double>&, int, bool);
 template void march_work<float>(const GridView<float>&, int, int, std::vector<int4>&);
 template void march_work<double>(const GridView<double>&, int, int, std::vector<int4>&);
 
