@@ -46,6 +46,20 @@ libFDTD.FDTD_mode_invert.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_void_p
 libFDTD.FDTD_mode_invert.restype = ctypes.c_int
 
 
+def _own_inverse(nb, n):
+    """Are n line blocks of nb rows inverted by FDTD_mode_invert, not by the
+    library?  Up to 640 rows always: the library is faster for a single block
+    only (606 rows, ms, own and library: 1 line 2.8 2.6, 2 lines 3.1 12.8, 80 lines
+    17.4 30.6).  Larger panels have fewer columns, so the update passes over the
+    matrix more often, and the library catches up with the number of lines: 900
+    rows 32 lines 30 41, 80 lines 69 65; 1280 rows 24 lines 56 67, 50 lines 107
+    97; 1400 rows 5 lines 30 50, 16 lines 72 66; 2400 rows 3 lines 79 91, 16 lines
+    339 186."""
+    if nb <= 640:
+        return True
+    return 2 <= n <= (45000 if nb <= 1280 else 10000) // nb
+
+
 def _check(rc, what):
     if rc != _ct.FDTD_OK:
         raise _ct.FDTDError("%s: %s" % (what, libFDTD.FDTD_mode_last_error().decode()))
@@ -201,16 +215,18 @@ class ModeFullVector:
             Lc[1:, ar, ar] = pval[1:][:, P_t]
             Uc[:-1, an, an] = nval[:-1][:, N_t]
 
-        # the blocks of a level's lines are inverted in place (FDTD_mode_invert);
-        # host tensors (tests) and blocks of more than 2560 rows go through torch
+        # the blocks of a level's lines are inverted in place (FDTD_mode_invert) where
+        # that is faster; host tensors (tests) and blocks of more than 2560 rows go
+        # through torch
         infos = []
-        work = int(libFDTD.FDTD_mode_invert_work(nb, NL)) if dev.type == "cuda" else 0
+        most = max((n for n in range(1, NL + 1) if _own_inverse(nb, n)), default=0)
+        work = int(libFDTD.FDTD_mode_invert_work(nb, most)) if dev.type == "cuda" and most else 0
         if work:
             work_t = torch.empty(work, dtype=torch.uint8, device=dev)
             stream = torch.cuda.current_stream(dev).cuda_stream
 
         def inv_into(lines, lines32):
-            if work:
+            if work and _own_inverse(nb, len(lines)):
                 info = torch.empty(len(lines), dtype=torch.int32, device=dev)
                 _check(libFDTD.FDTD_mode_invert(nb, self.device, stream, _ptr(D), _ptr(lines32), len(lines),
                                                 _ptr(work_t), work, _ptr(info)), "FDTD_mode_invert")
