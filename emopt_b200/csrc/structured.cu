@@ -30,7 +30,7 @@
 // 1e-14 of the cell area are dropped.  Overflow of either limit is reported.
 //
 // A layer's value at a cell does not depend on z, so one thread evaluates a
-// column of up to kPlanes cells and works each layer out once per column, not
+// column of up to kMaxPlanes cells and works each layer out once per column, not
 // once per cell: the geometry (four corner tests against every primitive of the
 // layer, and the clipping of the cells on an outline) bounds the cell-by-cell
 // form, the 16 bytes written per cell bound this one away from the outlines.
@@ -265,20 +265,23 @@ __device__ __forceinline__ void material_value(const Tables& t, double xd, doubl
     vr += (zmax - zmin) / dz * 1.0;
 }
 
-// Cells of a column per thread: short enough that a small grid fills the chip,
-// long enough that a layer is evaluated for many cells at a time.
-constexpr int kPlanes = 16;
+// Cells of a column per thread, chosen by the host: as many as leave 16 warps per
+// SM, so that a layer is evaluated for many cells at a time where there are many
+// cells, and no thread works alone through layer after layer of a small range.  us
+// at 16 cells and as chosen: 161 x 101 plane through 50 layers 274 -> 126, 48^3 cells
+// of 24 layers 386 -> 195, of 3 layers 84 -> 99; 5.2 M cells take 16 either way.
+constexpr int kMaxPlanes = 16;
 
 __global__ void __launch_bounds__(128) k_structured(Tables t, double dx, double dy, double dz, int k1,
                                                     int Nx, int j1, int i1, int Nz, long long cols,
                                                     double sx, double sy, double sz, c128* out,
-                                                    bool aligned, int* err) {
+                                                    bool aligned, int planes, int* err) {
     const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= cols) return;
     const int j = j1 + (int)(q / Nx);
     const int k = k1 + (int)(q % Nx);
     const double xd = (k + sx) * dx, yd = (j + sy) * dy;
-    const int a = (int)blockIdx.y * kPlanes, b = min(a + kPlanes, Nz);
+    const int a = (int)blockIdx.y * planes, b = min(a + planes, Nz);
     LayerCache c;
     int from = 0;
     for (int i = a; i < b; i++) {
@@ -401,13 +404,16 @@ extern "C" int FDTD_structured_values(int device, void* stream, const double* zs
         t.verts = reinterpret_cast<const double*>(px);
         fdtdb::c128* o = out_dev ? reinterpret_cast<fdtdb::c128*>(out) : dout;
         const long long cols = Nx * Ny;
+        int sms = 148;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+        const int planes = (int)std::min<long long>(fdtdb::kMaxPlanes, std::max<long long>(1, n / (sms * 16LL * 32)));
         // the y extent of a launch is bounded, so very deep ranges take several
-        const long long step = 65535LL * fdtdb::kPlanes;
+        const long long step = 65535LL * planes;
         for (long long i = 0; i < Nz && e == cudaSuccess; i += step) {
             const int nz = (int)std::min(step, Nz - i);
-            const dim3 grid((unsigned)((cols + 127) / 128), (unsigned)((nz + fdtdb::kPlanes - 1) / fdtdb::kPlanes));
+            const dim3 grid((unsigned)((cols + 127) / 128), (unsigned)((nz + planes - 1) / planes));
             fdtdb::k_structured<<<grid, 128, 0, st>>>(t, dx, dy, dz, k1, (int)Nx, j1, i1 + (int)i, nz, cols, sx, sy, sz,
-                                                      o + i * cols, (reinterpret_cast<uintptr_t>(o) & 15) == 0, perr);
+                                                      o + i * cols, (reinterpret_cast<uintptr_t>(o) & 15) == 0, planes, perr);
             e = cudaGetLastError();
         }
         if (e == cudaSuccess && !out_dev)
