@@ -198,6 +198,7 @@ extern "C" int FDTD_serve_admit(FDTDServe* s, FDTDHandle* h, const FDTDSolveOpti
     }
     Resident<float>& r = h->r32;
     auto hfail = [&]() { s->fail(h->status, "%s", h->message.c_str()); r.release_all(); return -h->status; };
+    r.release_second();     // of a solve of the handle by itself: not used here, not in the estimate
     if (alloc_resident<float>(h, r, h->w[0] + h->w[1]) != FDTD_OK) return hfail();
     if (prepare_materials<float>(h, r) != FDTD_OK) return hfail();
     fdtdb::SourceList<float> src;
