@@ -7,7 +7,7 @@ CUDA runtime statically, so it needs no torch or toolkit libraries at run time.
 
 A second library, ``emopt_b200/FDTD_checked.so``, is the same code with
 ``FDTD_BOUNDS_CHECK`` defined in the sources that hold the production
-stepping kernels (the vector pair and the serving kernel): every index those
+stepping kernels (the fused step, the vector pair and the serving kernel): every index those
 kernels compute is checked against its array, an out-of-range lane records
 where and skips the access, and the solve, slab and serving calls then fail
 with the site.  It is a debugging build, selected by setting
@@ -27,7 +27,7 @@ CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "FDTD.so")
 CHECKED = os.path.join(HERE, "FDTD_checked.so")
 # sources whose kernels carry the index checks in the checked library
-CHECKED_SOURCES = ["fdtd_abi.cu", "vec_kernels.cu", "serve_kernels.cu"]
+CHECKED_SOURCES = ["fdtd_abi.cu", "vec_kernels.cu", "zmarch_kernels.cu", "serve_kernels.cu"]
 BUILD = os.path.join(HERE, "_build")
 SOURCES = ["fdtd_abi.cu", "step_kernels.cu", "vec_kernels.cu", "zmarch_kernels.cu", "aux_kernels.cu",
            "legacy_kernels.cu", "grad_kernels.cu", "serve_kernels.cu", "noalloc.cu", "structured.cu",

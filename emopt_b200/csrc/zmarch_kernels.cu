@@ -151,6 +151,28 @@ __device__ __forceinline__ T* at(T* base, unsigned off) {
     return reinterpret_cast<T*>(reinterpret_cast<char*>(base) + off);
 }
 
+// Builds with FDTD_BOUNDS_CHECK: `want`, if the 16 bytes at offset off lie in an
+// array of `bytes`; else the site is recorded and the access left out.  (The box
+// copies need no check: what lies outside their arrays arrives as zeros.)
+template <typename T>
+__device__ __forceinline__ unsigned inside(const GridView<T>& g, unsigned want, unsigned off, long long bytes, int site) {
+#ifdef FDTD_BOUNDS_CHECK
+    return want && vecb::in_range(g, off, 0, bytes - 15, site) ? 1u : 0u;
+#else
+    return want;
+#endif
+}
+
+// ... and the local slab index l, if it is one of n; else -1.
+template <typename T>
+__device__ __forceinline__ int slab_inside(const GridView<T>& g, int l, int n, int site) {
+#ifdef FDTD_BOUNDS_CHECK
+    return l >= 0 && vecb::in_range(g, l, 0, n, site) ? l : -1;
+#else
+    return l;
+#endif
+}
+
 // Shared memory, in bytes.  Ex and Ez sit in a ring of three planes (the tile's
 // rows, the row below and the row above); everything else in two stages that
 // alternate by plane: Ey, H (with the row below), the E coefficients, the new
@@ -190,7 +212,7 @@ __device__ __forceinline__ void pair_load(const double* p, bool in, double& re, 
 // without branches between them, not one cell after the other (161 x 81 x 51 in
 // float32 with a 34 x 64 x 4 box of Jy and Mz: 27.7 -> 21.0 us a step).
 template <typename T, int BASE>
-__device__ __forceinline__ void vec_sources(const SourceList<T>& src, unsigned mask, int i, int j, int c0, T S, T C,
+__device__ __forceinline__ void vec_sources(const GridView<T>& g, const SourceList<T>& src, unsigned mask, int i, int j, int c0, T S, T C,
                                             pk::Vec<T>& a, pk::Vec<T>& b, pk::Vec<T>& c) {
     constexpr int VW = pk::Vec<T>::N;
     T f[3][VW];
@@ -199,6 +221,9 @@ __device__ __forceinline__ void vec_sources(const SourceList<T>& src, unsigned m
         const DevSource<T>& s = src.s[__ffs(mask) - 1];
         const int lk = c0 - s.k0;
         const long long m = 2 * (((long long)(i - s.i0) * s.J + (j - s.j0)) * s.K + lk);
+#ifdef FDTD_BOUNDS_CHECK
+        if (!vecb::in_range(g, i, s.i0, s.i0 + s.I, 27) || !vecb::in_range(g, j, s.j0, s.j0 + s.J, 27)) continue;
+#endif
 #pragma unroll
         for (int q = 0; q < 3; q++) {
             const T* p = s.comp[BASE + q];
@@ -283,6 +308,11 @@ k_step_march(const __grid_constant__ MarchArgs<T> A, const __grid_constant__ Sou
     const int x0 = job.x * (30 * VW), c0 = x0 + lane * VW;
     const int j0 = job.y * R, j = j0 - 1 + w;
     const int i0 = job.z, i1 = job.w, is = i0 > 0 ? i0 - 1 : 0;
+#ifdef FDTD_BOUNDS_CHECK
+    if (!vecb::in_range(g, x0, 0, g.Nx, 20) || !vecb::in_range(g, job.y * R, 0, g.Ny, 20) ||
+        !vecb::in_range(g, i0, 0, i1, 20) || !vecb::in_range(g, i1, 1, g.Nz + 1, 20))
+        return;
+#endif
     const bool row = j >= 0 && j < g.Ny;
     const bool ok = row && c0 < g.Nx;
     const bool own = ok && w > 0 && (lane > 0 || job.x == 0) && (lane < 31 || job.x == A.x_tiles - 1);
@@ -290,7 +320,7 @@ k_step_march(const __grid_constant__ MarchArgs<T> A, const __grid_constant__ Sou
     const unsigned pb = (unsigned)g.Ny * g.px * SZ;
     const unsigned rb = ok ? (unsigned)(j * g.px + c0) * SZ : 0u;
     const unsigned sbase = smem_u32(smem);
-    const int ly = row ? slab_local(PY, j, false) : -1;
+    const int ly = slab_inside(g, row ? slab_local(PY, j, false) : -1, PY.wsum, 22);
     // x slab: slot of this vector in the whole-vector psi rows, or -1
     int sx = -1;
     if (c0 < PX.w0) sx = c0;
@@ -389,7 +419,10 @@ k_step_march(const __grid_constant__ MarchArgs<T> A, const __grid_constant__ Sou
     if (threadIdx.x == 32) sh_store<0>(sbase + L::zero, V::zero());
     const unsigned xta = sbase + L::xt + lane * 16;
     V ey = V::zero(), hpy = V::zero();      // Ey of the plane, new Hy of the plane below
-    if (ok) ey = V::load(at(A.in.c[1], (unsigned)is * pb + rb));
+    // array sizes of the checked build: fields, x-, y- and z-slab state
+    const long long fbytes = (long long)g.Nz * pb, xbytes_all = (long long)g.Nz * g.Ny * A.x_pitch * SZ;
+    const long long ybytes = (long long)g.Nz * PY.wsum * g.px * SZ, zbytes = (long long)PZ.wsum * pb;
+    if (inside(g, ok, (unsigned)is * pb + rb, fbytes, 21)) ey = V::load(at(A.in.c[1], (unsigned)is * pb + rb));
     __syncthreads();
 
     const bool iny = ly >= 0, xmin = job.x == 0;
@@ -405,15 +438,21 @@ k_step_march(const __grid_constant__ MarchArgs<T> A, const __grid_constant__ Sou
 
 #pragma unroll 1
     for (int i = is; i < i1; i++) {
-        const int lz = slab_local(PZ, i + PZ.off, true);
+        const int lz = slab_inside(g, slab_local(PZ, i + PZ.off, true), PZ.wsum, 23);
         const bool inz = lz >= 0, emit = i >= i0;      // the plane before the chunk: H only
         const unsigned oZ = (unsigned)lz * pb + rb;
-        const unsigned eo = emit ? ownu : 0u, eox = emit ? ownxu : 0u;
+        const unsigned eo = inside(g, emit ? ownu : 0u, o, fbytes, 21), eox = inside(g, emit ? ownxu : 0u, oX, xbytes_all, 24);
 
         // ---- CPML state of the H update
         V py0, py1, pz0, pz1;
-        if (iny) { py0 = gload(at(A.ph_in[1][0], oY), 1u); py1 = gload(at(A.ph_in[1][1], oY), 1u); }
-        if (inz) { pz0 = gload(at(A.ph_in[2][0], oZ), 1u); pz1 = gload(at(A.ph_in[2][1], oZ), 1u); }
+        if (iny) {
+            const unsigned in = inside(g, 1u, oY, ybytes, 25);
+            py0 = gload(at(A.ph_in[1][0], oY), in); py1 = gload(at(A.ph_in[1][1], oY), in);
+        }
+        if (inz) {
+            const unsigned in = inside(g, 1u, oZ, zbytes, 26);
+            pz0 = gload(at(A.ph_in[2][0], oZ), in); pz1 = gload(at(A.ph_in[2][1], oZ), in);
+        }
 
         // ---- which cells round their curls as the vector pair's plain body;
         // the sources of this row in this plane
@@ -452,8 +491,8 @@ k_step_march(const __grid_constant__ MarchArgs<T> A, const __grid_constant__ Sou
             const V fzdx = ez.diff_down(), fydx = ey.diff_down(), fxdy = pk::sub(exj, ex);
             V m0, m1, m2;
             if (MUARR) {
-                m0 = gload(at(g.bHarr[0], o), ok ? 1u : 0u); m1 = gload(at(g.bHarr[1], o), ok ? 1u : 0u);
-                m2 = gload(at(g.bHarr[2], o), ok ? 1u : 0u);
+                const unsigned in = inside(g, ok ? 1u : 0u, o, fbytes, 21);
+                m0 = gload(at(g.bHarr[0], o), in); m1 = gload(at(g.bHarr[1], o), in); m2 = gload(at(g.bHarr[2], o), in);
             } else {
                 m0 = V::dup(A.m[0]); m1 = V::dup(A.m[1]); m2 = V::dup(A.m[2]);
             }
@@ -471,7 +510,8 @@ k_step_march(const __grid_constant__ MarchArgs<T> A, const __grid_constant__ Sou
                     p0 = sh_load<T, 0>(q);
                     p1 = sh_load<T, 0>(sxu ? q + NW * kXRow : q);
                 } else {
-                    p0 = gload(at(A.ph_in[0][0], oX), sxu); p1 = gload(at(A.ph_in[0][1], oX), sxu);
+                    const unsigned in = inside(g, sxu, oX, xbytes_all, 24);
+                    p0 = gload(at(A.ph_in[0][0], oX), in); p1 = gload(at(A.ph_in[0][1], oX), in);
                 }
                 hz = pk::fnma(m2, cpml(p0, pk::mul(ox, fydx), kv, bv, cv, mone), hz);
                 hy = pk::fma(m1, cpml(p1, pk::mul(ox, fzdx), kv, bv, cv, mone), hy);
@@ -481,16 +521,18 @@ k_step_march(const __grid_constant__ MarchArgs<T> A, const __grid_constant__ Sou
                 const Coef<T> c = coef<T>(A.ytab + 6 * ly);
                 hz = pk::fma(m2, cpml(py0, pk::mul(oy, fxdy), c.k, c.b, c.c, mone), hz);
                 hx = pk::fnma(m0, cpml(py1, pk::mul(oy, fzdy), c.k, c.b, c.c, mone), hx);
-                gstore(at(A.ph_out[1][0], oY), py0, eo); gstore(at(A.ph_out[1][1], oY), py1, eo);
+                const unsigned in = inside(g, eo, oY, ybytes, 25);
+                gstore(at(A.ph_out[1][0], oY), py0, in); gstore(at(A.ph_out[1][1], oY), py1, in);
             }
             if (inz) {
                 const Coef<T> c = coef<T>(A.ztab + 6 * lz);
                 hx = pk::fma(m0, cpml(pz1, pk::mul(oz, fydz), c.k, c.b, c.c, mone), hx);
                 hy = pk::fnma(m1, cpml(pz0, pk::mul(oz, fxdz), c.k, c.b, c.c, mone), hy);
-                gstore(at(A.ph_out[2][0], oZ), pz0, eo); gstore(at(A.ph_out[2][1], oZ), pz1, eo);
+                const unsigned in = inside(g, eo, oZ, zbytes, 26);
+                gstore(at(A.ph_out[2][0], oZ), pz0, in); gstore(at(A.ph_out[2][1], oZ), pz1, in);
             }
         }
-        if (now & 0xffffu) vec_sources<T, 3>(src, now & 0xffffu, i, j, c0, srcS[0], srcC[0], hx, hy, hz);
+        if (now & 0xffffu) vec_sources<T, 3>(g, src, now & 0xffffu, i, j, c0, srcS[0], srcC[0], hx, hy, hz);
         sh_store<L::x>(sa, hx);
         sh_store<L::x + NW * kRow>(sa, hz);
         gstore(at(A.out.c[3], o), hx, eo);
@@ -498,8 +540,14 @@ k_step_march(const __grid_constant__ MarchArgs<T> A, const __grid_constant__ Sou
         gstore(at(A.out.c[5], o), hz, eo);
 
         // ---- CPML state of the E update
-        if (iny) { py0 = gload(at(A.pe[1][0], oY), eo); py1 = gload(at(A.pe[1][1], oY), eo); }
-        if (inz) { pz0 = gload(at(A.pe[2][0], oZ), eo); pz1 = gload(at(A.pe[2][1], oZ), eo); }
+        if (iny) {
+            const unsigned in = inside(g, eo, oY, ybytes, 25);
+            py0 = gload(at(A.pe[1][0], oY), in); py1 = gload(at(A.pe[1][1], oY), in);
+        }
+        if (inz) {
+            const unsigned in = inside(g, eo, oZ, zbytes, 26);
+            pz0 = gload(at(A.pe[2][0], oZ), in); pz1 = gload(at(A.pe[2][1], oZ), in);
+        }
         V a0, a1, a2;                                  // E-update factors of lossy media
         if (LOSSY) { a0 = gload(at(g.aE[0], o), eo); a1 = gload(at(g.aE[1], o), eo); a2 = gload(at(g.aE[2], o), eo); }
         __syncthreads();
@@ -564,28 +612,33 @@ k_step_march(const __grid_constant__ MarchArgs<T> A, const __grid_constant__ Sou
                         p0 = sh_load<T, 0>(q);
                         p1 = sh_load<T, 0>(sxu ? q + NW * kXRow : q);
                     } else {
-                        p0 = gload(at(A.pe[0][0], oX), ownxu); p1 = gload(at(A.pe[0][1], oX), ownxu);
+                        const unsigned in = inside(g, ownxu, oX, xbytes_all, 24);
+                        p0 = gload(at(A.pe[0][0], oX), in); p1 = gload(at(A.pe[0][1], oX), in);
                     }
                     ez = pk::fma(cpml(p0, pk::mul(ox, fydx), kv, bv, cv, mone), bz, ez);
                     ey = pk::fnma(cpml(p1, pk::mul(ox, fzdx), kv, bv, cv, mone), by, ey);
-                    gstore(at(A.pe[0][0], oX), p0, ownxu); gstore(at(A.pe[0][1], oX), p1, ownxu);
+                    const unsigned in = inside(g, ownxu, oX, xbytes_all, 24);
+                    gstore(at(A.pe[0][0], oX), p0, in); gstore(at(A.pe[0][1], oX), p1, in);
                 }
                 if (iny) {
                     const Coef<T> c = coef<T>(A.ytab + 6 * ly + 3);
                     ez = pk::fnma(cpml(py0, pk::mul(oy, fxdy), c.k, c.b, c.c, mone), bz, ez);
                     ex = pk::fma(cpml(py1, pk::mul(oy, fzdy), c.k, c.b, c.c, mone), bx, ex);
-                    gstore(at(A.pe[1][0], oY), py0, ownu); gstore(at(A.pe[1][1], oY), py1, ownu);
+                    const unsigned in = inside(g, ownu, oY, ybytes, 25);
+                    gstore(at(A.pe[1][0], oY), py0, in); gstore(at(A.pe[1][1], oY), py1, in);
                 }
                 if (inz) {
                     const Coef<T> c = coef<T>(A.ztab + 6 * lz + 3);
                     ex = pk::fnma(cpml(pz1, pk::mul(oz, fydz), c.k, c.b, c.c, mone), bx, ex);
                     ey = pk::fma(cpml(pz0, pk::mul(oz, fxdz), c.k, c.b, c.c, mone), by, ey);
-                    gstore(at(A.pe[2][0], oZ), pz0, ownu); gstore(at(A.pe[2][1], oZ), pz1, ownu);
+                    const unsigned in = inside(g, ownu, oZ, zbytes, 26);
+                    gstore(at(A.pe[2][0], oZ), pz0, in); gstore(at(A.pe[2][1], oZ), pz1, in);
                 }
-                if (now >> 16) vec_sources<T, 0>(src, now >> 16, i, j, c0, srcS[1], srcC[1], ex, ey, ez);
-                gstore(at(A.out.c[0], o), ex, ownu);
-                gstore(at(A.out.c[1], o), ey, ownu);
-                gstore(at(A.out.c[2], o), ez, ownu);
+                if (now >> 16) vec_sources<T, 0>(g, src, now >> 16, i, j, c0, srcS[1], srcC[1], ex, ey, ez);
+                const unsigned in = inside(g, ownu, o, fbytes, 21);
+                gstore(at(A.out.c[0], o), ex, in);
+                gstore(at(A.out.c[1], o), ey, in);
+                gstore(at(A.out.c[2], o), ez, in);
             }
         }
         ey = eyi;
