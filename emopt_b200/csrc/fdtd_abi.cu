@@ -1054,7 +1054,7 @@ int prepare_sources(FDTDHandle* h, Resident<T>& r, fdtdb::SourceList<T>& list) {
 }
 
 template <typename T>
-fdtdb::GridView<T> make_view(FDTDHandle* h, Resident<T>& r, int set = 0) {
+fdtdb::GridView<T> make_view(FDTDHandle* h, Resident<T>& r) {
     fdtdb::GridView<T> g;
     g.Nx = h->Nx; g.Ny = h->Ny; g.Nz = h->Nz; g.px = r.px;
     g.plane = (long long)h->Ny * r.px;
@@ -1072,7 +1072,7 @@ fdtdb::GridView<T> make_view(FDTDHandle* h, Resident<T>& r, int set = 0) {
         P.w0 = h->w[2 * a]; P.w1 = h->w[2 * a + 1]; P.wsum = P.w0 + P.w1;
         P.edge_max = N[a] - P.w1;
         P.off = 0;
-        for (int q = 0; q < 4; q++) P.psi[q] = dptr<T>(r.psi[set][a][q]);
+        for (int q = 0; q < 4; q++) P.psi[q] = dptr<T>(r.psi[0][a][q]);
         P.kinvH = dptr<T>(r.tab[a][0]); P.bH = dptr<T>(r.tab[a][1]);
         P.cH = dptr<T>(r.tab[a][2]); P.kinvE = dptr<T>(r.tab[a][3]);
         P.bE = dptr<T>(r.tab[a][4]); P.cE = dptr<T>(r.tab[a][5]);
@@ -1090,7 +1090,7 @@ fdtdb::GridView<T> make_view(FDTDHandle* h, Resident<T>& r, int set = 0) {
 // The fused step's view of the resident state: reads field set `set`.
 template <typename T>
 int make_march(FDTDHandle* h, Resident<T>& r, int set, bool src_general, fdtdb::MarchArgs<T>& a) {
-    a.g = make_view<T>(h, r, 0);
+    a.g = make_view<T>(h, r);
     for (int c = 0; c < 6; c++) {
         a.in.c[c] = dptr<T>(r.F[set][c]);
         a.out.c[c] = dptr<T>(r.F[1 - set][c]);
@@ -1188,7 +1188,7 @@ int solve_impl(FDTDHandle* h, const FDTDSolveOptions* o, FDTDSolveResult* res) {
     // place (src_general), so that choice changes no bit.
     bool split_rule = false;
     if (sizeof(T) == 4 && !periodic && small_index)
-        split_rule = fdtdb::split_interior_fraction<T>(make_view<T>(h, r, 0)) >= 0.6;
+        split_rule = fdtdb::split_interior_fraction<T>(make_view<T>(h, r)) >= 0.6;
     int kid = h->kernel;
     const int pair = periodic || !small_index ? 1 : split_rule ? 6 : 5;
     int dev_sms = 148;
@@ -1286,7 +1286,7 @@ int solve_impl(FDTDHandle* h, const FDTDSolveOptions* o, FDTDSolveResult* res) {
     pd.nconv = nconv;
 
     long long* sb = dptr<long long>(r.stepbase);
-    fdtdb::GridView<T> g0 = make_view<T>(h, r, 0);
+    fdtdb::GridView<T> g0 = make_view<T>(h, r);
     fdtdb::MarchArgs<T> m0, m1;
     if (fused) {
         if ((rc = make_march<T>(h, r, 0, !split_rule, m0)) != FDTD_OK) return rc;

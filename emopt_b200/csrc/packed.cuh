@@ -47,12 +47,7 @@ struct Vec<float> {
     static __device__ __forceinline__ void unpack(unsigned long long r, float& a, float& b) {
         asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r));
     }
-    static __device__ __forceinline__ Vec bcast(float a) {
-        Vec r;
-        r.v[0] = r.v[1] = pack(a, a);
-        return r;
-    }
-    // a pair of equal values (Dup<float>)
+    // a pair of equal values (DupOf<float>)
     static __device__ __forceinline__ Vec dup(unsigned long long a) {
         Vec r;
         r.v[0] = r.v[1] = a;
@@ -69,9 +64,6 @@ struct Vec<float> {
         r.v[0] = q.x;
         r.v[1] = q.y;
         return r;
-    }
-    __device__ __forceinline__ void store(float* p) const {
-        *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(v[0], v[1]);
     }
     __device__ __forceinline__ void get(float* f) const {
         unpack(v[0], f[0], f[1]);
@@ -129,9 +121,6 @@ struct Vec<double> {
         r.v[1] = q.y;
         return r;
     }
-    __device__ __forceinline__ void store(double* p) const {
-        *reinterpret_cast<double2*>(p) = make_double2(v[0], v[1]);
-    }
     __device__ __forceinline__ void get(double* f) const { f[0] = v[0]; f[1] = v[1]; }
     __device__ __forceinline__ void set(const double* f) { v[0] = f[0]; v[1] = f[1]; }
     __device__ __forceinline__ double at0() const { return v[0]; }
@@ -166,7 +155,6 @@ struct Vec<double> {
         r.v[1] = scalar(a.v[1], b.v[1]);                                                                   \
         return r;                                                                                          \
     }
-PK_OP2(add, "add.rn.f32x2", __dadd_rn)
 PK_OP2(sub, "sub.rn.f32x2", __dsub_rn)
 PK_OP2(mul, "mul.rn.f32x2", __dmul_rn)
 #undef PK_OP2
