@@ -20,17 +20,18 @@
 // both publishes them and frees the ring slots the next copies overwrite.
 //
 // What bounds it: without CPML DRAM (321 x 161 x 101 cells in float32: 71 us a
-// step, 313 MB; 4.4 TB/s); with 20-cell slabs the latency of a plane, 4000
-// cycles for a CTA in no slab and 6500-9000 in one to three of them, of which
-// the slab state read from DRAM is the largest part.  16 warps per SM is what
-// 113 KB of shared memory and 128 registers leave, and any register spilled
-// inside the plane loop costs more than it saves (the L1 is all shared memory:
-// 16 bytes spilled took 193 us instead of 126).  us per step, before (vector
-// pair, in the large slab the interior/rim pair) and now, 10- to 20-cell slabs:
-//   float32  80x80x80 24.9 -> 17.2, 161x81x51 22.9 -> 19.1, 321x161x101 122.8 ->
-//            104.4, 801x401x201 1043 -> 905
-//   float64  101x76x65 27.0 -> 23.9, 161x81x51 28.9 -> 27.7, 321x161x101 207.5 ->
-//            184.7
+// step, 313 MB; 4.4 TB/s); with 20-cell slabs the latency of a plane, 3650
+// cycles for a CTA in no slab and up to 8300 in all three of them, of which the
+// slab state read from DRAM is the largest part.  16 warps per SM is what 112 KB
+// of shared memory and 128 registers (120 lossless in float32) leave, and any
+// register spilled inside the plane loop costs more than it saves (the L1 is all
+// shared memory: 16 bytes spilled took 193 us instead of 126).  us per step,
+// before (vector pair, in the large slab the interior/rim pair) and now, 10- to
+// 20-cell slabs, a line of current (801x401x201: a plane):
+//   float32  80x80x80 24.9 -> 15.3, 161x81x51 22.1 -> 17.3, 321x161x101 121.6 ->
+//            100.7, 801x401x201 1043 -> 905
+//   float64  101x76x65 26.8 -> 22.5, 161x81x51 27.0 -> 25.2, 321x161x101 205.0 ->
+//            181.8
 // Steps are launched with programmatic serialization: a step's CTAs start up in
 // the slots the last CTAs of the step before leave and wait there for its end
 // (16.6 -> 14.4 us on 64x64x64, 21.2 -> 20.0 on 161x81x51 in float32, 920 -> 905

@@ -122,15 +122,16 @@ int FDTD_set_zchunk(FDTDHandle *h, int planes);
 int FDTD_set_precision(FDTDHandle *h, int bits);
 
 /* Time-stepping kernel of FDTD_solve_cw: 0 = automatic (default: 3 where
- * rows hold more than 16 vectors of 16 bytes, no axis is periodic and the
- * second set of fields fits in memory; else 6 in float32 when at least 60% of
+ * rows hold more than 16 vectors of 16 bytes, no axis is periodic, the grid's
+ * shape lets it be the faster one and the second set of fields fits in memory
+ * beside everything else the solve needs; else 6 in float32 when at least 60% of
  * the 64-cell warp tasks lie in no CPML slab; else 5), 1 = H and E kernels
  * with one cell per thread, 3 = one fused H+E kernel per time step whose
  * CTAs march up z chunks (reads one field/CPML set, writes the other), 5 = H
  * and E kernels with one 2-element vector of x cells per thread, 6 = the
  * kernels of 5 split per half step into an interior launch (tasks in no CPML
- * slab) and a rim launch.  3, 5 and 6 give the same bits where auto chooses
- * among them.  Other values fail with FDTD_ERR_ARG.  Periodic boundaries
+ * slab) and a rim launch.  3 gives the bits of the pair (5 or 6) that auto
+ * takes in its place; 5 and 6 differ in float32 by rounding next to sources.  Other values fail with FDTD_ERR_ARG.  Periodic boundaries
  * always use 1. */
 int FDTD_set_kernel(FDTDHandle *h, int which);
 
